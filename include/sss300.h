@@ -101,7 +101,9 @@ typedef struct sss_tof_problem {
     const float *atten_ratio;      /* device, [2000]: water mu(E)/mu(511) (:117-120) */
     int32_t flags;                 /* SSS_FLAG_*; 0 = the plain FP32 reduction */
     int32_t pair_warps;            /* launch shape (no reference counterpart): warps per pair-kernel
-                                      block, 0 = sss_pair_warps_max(nbins, flags), else 1..that */
+                                      block, 0 = sss_pair_warps_max(nbins, flags), else 1..that; the
+                                      histogram kernel of several TOF bins takes it as a share of
+                                      its own largest block */
     int32_t leg_threads;           /* threads per leg-kernel block, 0 = 128, else a multiple of 32
                                       up to 256 */
 } sss_tof_problem;

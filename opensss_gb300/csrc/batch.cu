@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "hist.cuh"
 #include "legs.cuh"
 #include "pair.cuh"
 #include "trace.cuh"
@@ -161,18 +162,25 @@ LatticeSize lattice_size(const sss_tof_problem& p)
 }
 
 // leg-record bytes of `npts` scatter points of problem p
-size_t item_bytes(const sss_tof_problem& p, long long npts)
+size_t item_bytes(const sss_tof_problem& p, long long npts, bool hist)
 {
     const long long nl = (long long)p.nru * p.ndu;
     const long long cap = (long long)p.nx + p.ny + p.nz;
     const size_t lists = (p.flags & SSS_FLAG_UNIT_TOF) ? 0 : align256(sizeof(float2) * npts * nl * cap);
-    return 3 * align256(sizeof(float4) * npts * nl) + lists;
+    size_t bytes = 3 * align256(sizeof(float4) * npts * nl) + lists;
+    if (hist && hist_lists(p)) {
+        const FactorSize f = factor_size(p, npts, 1);
+        bytes += align256(sizeof(float4) * npts * nl) + align256(f.c) + align256(f.inv) + align256(f.zeroed);
+    }
+    return bytes;
 }
 
 }  // namespace
 
 struct sss_batch {
     struct Launch {
+        bool hist = false;      // the histogram pair stage (launch in hl), else the direct one below
+        HistLaunch hl;
         int nbins;
         TofConst T;
         const float* tof;
@@ -190,6 +198,7 @@ struct sss_batch {
         long long threads;
         int ctr_first;          // the wave's launch counters: counters[ctr_first ..]
         std::vector<Launch> launches;
+        std::vector<std::pair<char*, size_t>> clear;  // zeroed before the pair launches
     };
     std::vector<sss_tof_problem> problems;
     std::vector<float*> outs;
@@ -226,6 +235,10 @@ int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
                const std::vector<const double*>& points,
                const std::vector<std::vector<unsigned long long>>& counts, char* ws, size_t off,
                size_t workspace_bytes, int32_t* status, sss_batch** plan, cudaStream_t st);
+int plan_form(const sss_tof_problem* problems, int32_t n, float* const* outs,
+              const std::vector<const double*>& points,
+              const std::vector<std::vector<unsigned long long>>& counts, char* ws, size_t off,
+              size_t workspace_bytes, int32_t* status, sss_batch** plan, cudaStream_t st, bool hist);
 
 }  // namespace
 
@@ -310,11 +323,30 @@ extern "C" int sss_batch_plan_points(const sss_tof_problem* problems, int32_t n,
 
 namespace {
 
+using TofClass = std::tuple<int, double, double>;  // bins, bin width, resolution
+TofClass tof_class(const sss_tof_problem& p) { return TofClass(p.nbins, p.tof_bin_width, p.tof_resolution); }
+
+// The histogram pair stage needs TOF rows per class, the pairs' factors of a
+// wave and a record more per leg.  A workspace in which a z-slice does not fit
+// with them is planned with the direct kernels instead, which evaluate the
+// weights voxel by voxel and need nothing beside the leg records.
 int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
                const std::vector<const double*>& points,
                const std::vector<std::vector<unsigned long long>>& counts, char* ws, size_t off,
                size_t workspace_bytes, int32_t* status, sss_batch** plan, cudaStream_t st)
 {
+    int rc = plan_form(problems, n, outs, points, counts, ws, off, workspace_bytes, status, plan, st, true);
+    if (rc == SSS_ERR_WORKSPACE)
+        rc = plan_form(problems, n, outs, points, counts, ws, off, workspace_bytes, status, plan, st, false);
+    return rc;
+}
+
+int plan_form(const sss_tof_problem* problems, int32_t n, float* const* outs,
+              const std::vector<const double*>& points,
+              const std::vector<std::vector<unsigned long long>>& counts, char* ws, size_t off,
+              size_t workspace_bytes, int32_t* status, sss_batch** plan, cudaStream_t st, bool hist)
+{
+    const size_t off0 = off;
     auto take = [&](size_t bytes) {
         size_t o = off;
         off = align256(off + bytes);
@@ -348,6 +380,20 @@ int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
     const size_t pdesc_off = take(sizeof(PairItem) * std::max<size_t>(items.size(), 1));
     const int max_launches = (int)items.size() + 1;
     const size_t ctr_off = take(sizeof(unsigned int) * (size_t)max_launches);
+    // the histogram form: runs of slices, their point counts, TOF rows, flush partials
+    size_t seg_off = 0, slice_off = 0, partial_off = 0;
+    std::map<TofClass, size_t> rows_off;
+    if (hist) {
+        seg_off = take(sizeof(HistSeg) * std::max<size_t>(items.size(), 1));
+        slice_off = take(sizeof(int32_t) * 2 * std::max<size_t>(items.size(), 1));
+        for (const Item& it : items) {
+            const sss_tof_problem& p = problems[it.prob];
+            if (hist_lists(p) && !rows_off.count(tof_class(p))) rows_off[tof_class(p)] = take(hist_rows_bytes(p.nbins));
+        }
+        if (!rows_off.empty()) partial_off = take(hist_partial_bytes());
+        if (off - off0 > (workspace_bytes - off0) / 2)
+            return sss_set_error(SSS_ERR_WORKSPACE, "sss_batch_plan: no room for the histogram form");
+    }
     const size_t data_off = off;
     if (data_off >= workspace_bytes)
         return sss_set_error(SSS_ERR_WORKSPACE, "sss_batch_plan: no workspace left for leg records");
@@ -358,13 +404,19 @@ int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
     std::vector<PairItem> hpair(items.size());
     LegItem* dleg = (LegItem*)(ws + desc_off);
     PairItem* dpair = (PairItem*)(ws + pdesc_off);
+    std::vector<HistSeg> hseg(hist ? items.size() : 0);
+    std::vector<FactorOut> hfac(items.size());
+    std::vector<int32_t> hslice(hist ? 2 * items.size() : 0);
+    HistSeg* dseg = (HistSeg*)(ws + seg_off);
+    int32_t* dslice = (int32_t*)(ws + slice_off);
+    size_t nseg = 0, nslice = 0;
     unsigned int* dctr = (unsigned int*)(ws + ctr_off);
     int nctr = 0;
     size_t k = 0;
     while (k < items.size()) {
         size_t used = 0, k_end = k;
         while (k_end < items.size()) {
-            const size_t b = item_bytes(problems[items[k_end].prob], items[k_end].count);
+            const size_t b = item_bytes(problems[items[k_end].prob], items[k_end].count, hist);
             if (used + b > data_bytes) break;
             used += b;
             ++k_end;
@@ -373,7 +425,7 @@ int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
             return sss_set_error(SSS_ERR_WORKSPACE,
                                  "sss_batch_plan: a z-slice of problem %d needs %zu bytes of leg records, "
                                  "only %zu available", items[k].prob,
-                                 item_bytes(problems[items[k].prob], items[k].count), data_bytes);
+                                 item_bytes(problems[items[k].prob], items[k].count, hist), data_bytes);
         sss_batch::Wave W;
         W.ctr_first = nctr;
         W.legs = dleg + k;
@@ -381,7 +433,10 @@ int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
         W.threads = 0;
         size_t doff = data_off;
         // group the wave's items by TOF class for the pair launches
-        std::map<std::tuple<int, double, double>, std::vector<size_t>> classes;
+        std::map<TofClass, std::vector<size_t>> classes;
+        long long run_first = 0;
+        float4 *rA = nullptr, *rB = nullptr, *rC = nullptr, *rD = nullptr;
+        float2* rV = nullptr;
         for (size_t j = k; j < k_end; ++j) {
             const Item& it = items[j];
             const sss_tof_problem& p = problems[it.prob];
@@ -403,23 +458,42 @@ int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
             L.p.nvox = (long long)p.nx * p.ny * p.nz;
             L.p.points = points[it.prob] + 4 * it.first;
             L.p.npts = (int)it.count;
-            L.p.legA = (float4*)(ws + doff);
-            doff += align256(sizeof(float4) * it.count * nl);
-            L.p.legB = (float4*)(ws + doff);
-            doff += align256(sizeof(float4) * it.count * nl);
-            L.p.legC = (float4*)(ws + doff);
-            doff += align256(sizeof(float4) * it.count * nl);
-            if (p.flags & SSS_FLAG_UNIT_TOF) {
-                L.p.vox = nullptr;  // every TOF weight is 1: the pairs use the leg integrals
-            } else {
-                L.p.vox = (float2*)(ws + doff);
-                doff += align256(sizeof(float2) * it.count * nl * cap);
+            if (j == k || items[j - 1].prob != it.prob) {
+                // a run: the wave's slices of one problem, their records contiguous
+                run_first = it.first;
+                long long pts = 0;
+                for (size_t m = j; m < k_end && items[m].prob == it.prob; ++m) pts += items[m].count;
+                auto run = [&](size_t bytes) {
+                    char* at = ws + doff;
+                    doff += align256(bytes);
+                    return at;
+                };
+                rA = (float4*)run(sizeof(float4) * pts * nl);
+                rB = (float4*)run(sizeof(float4) * pts * nl);
+                rC = (float4*)run(sizeof(float4) * pts * nl);
+                rD = hist && hist_lists(p) ? (float4*)run(sizeof(float4) * pts * nl) : nullptr;
+                if (rD) {
+                    long long slices = 0;
+                    for (size_t m = j; m < k_end && items[m].prob == it.prob; ++m) ++slices;
+                    const FactorSize f = factor_size(p, pts, slices);
+                    char *fc = run(f.c), *fi = run(f.inv), *fz = run(f.zeroed);
+                    hfac[j] = factor_out(p, fc, fi, fz);
+                    W.clear.push_back({fz, f.zeroed});
+                }
+                // unit TOF weights: no lists, the pairs use the leg integrals
+                rV = (p.flags & SSS_FLAG_UNIT_TOF) ? nullptr : (float2*)run(sizeof(float2) * pts * nl * cap);
             }
+            const long long at = (it.first - run_first) * nl;
+            L.p.legA = rA + at;
+            L.p.legB = rB + at;
+            L.p.legC = rC + at;
+            L.p.legD = rD ? rD + at : nullptr;
+            L.p.vox = rV ? rV + at * cap : nullptr;
             L.p.vox_lo = nullptr;
             L.p.status = status;
             L.thread_begin = W.threads;
             W.threads += it.count * nl;
-            classes[std::make_tuple(p.nbins, p.tof_bin_width, p.tof_resolution)].push_back(j);
+            classes[tof_class(p)].push_back(j);
         }
         // pair items, contiguous per class
         size_t pk = k;
@@ -433,14 +507,9 @@ int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
             Lc.nitems = (int)kv.second.size();
             Lc.ntasks = 0;
             Lc.counter = dctr + nctr++;
-            Lc.fn = pick_batch_pairs(p0.nbins);
-            Lc.warps = p0.pair_warps ? p0.pair_warps : pair_block_warps((p0.nbins + 1) / 2, false);
-            if (!Lc.fn) return sss_set_error(SSS_ERR_INVALID, "sss_batch_plan: nbins out of range");
-            for (size_t j : kv.second) {
-                const Item& it = items[j];
-                const sss_tof_problem& p = problems[it.prob];
-                PairItem& P = hpair[pk++];
-                PairCtx& C = P.ctx;
+            auto context = [&](size_t j) {
+                const sss_tof_problem& p = problems[items[j].prob];
+                PairCtx C;
                 C.nru = p.nru;
                 C.ndu = p.ndu;
                 C.nl = p.nru * p.ndu;
@@ -458,14 +527,71 @@ int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
                 C.legA = hleg[j].p.legA;
                 C.legB = hleg[j].p.legB;
                 C.legC = hleg[j].p.legC;
+                C.legD = hleg[j].p.legD;
                 C.vox = hleg[j].p.vox;
-                C.vox_lo = nullptr;  // the batched engine runs the plain pair kernel
+                C.vox_lo = nullptr;  // the precision launch is not part of the batched engine
                 C.unit_tof = (p.flags & SSS_FLAG_UNIT_TOF) != 0;
-                C.out = outs[it.prob];
+                C.out = outs[items[j].prob];
+                return C;
+            };
+            // a class of one bin can mix unit and varying weights: those run direct
+            Lc.hist = hist;
+            for (size_t j : kv.second)
+                Lc.hist = Lc.hist && hist_form(problems[items[j].prob]) &&
+                          hist_lists(problems[items[j].prob]) == hist_lists(p0);
+            if (Lc.hist) {
+                HistLaunch& H = Lc.hl;
+                H = HistLaunch();
+                H.unit = !hist_lists(p0);
+                H.segs = dseg + nseg;
+                H.counter = Lc.counter;
+                H.status = status;
+                H.partial = (float*)(ws + partial_off);
+                for (size_t m = 0; m < kv.second.size();) {
+                    const size_t j = kv.second[m];
+                    const sss_tof_problem& p = problems[items[j].prob];
+                    HistSeg& G = hseg[nseg++];
+                    G.ctx = context(j);
+                    H.most_legs = std::max(H.most_legs, G.ctx.nl);
+                    G.rows = H.unit ? nullptr : (const float*)(ws + rows_off[kv.first]);
+                    G.f = hfac[j];
+                    G.first = dslice + nslice;
+                    size_t e = m;
+                    long long pts = 0;
+                    for (; e < kv.second.size() && items[kv.second[e]].prob == items[j].prob; ++e)
+                        pts += items[kv.second[e]].count;
+                    hist_shape(p, (int)(e - m), (int)pts, G);
+                    G.count = G.first + G.nslices;
+                    for (int z = 0; z < G.nslices; ++z) {
+                        const Item& it = items[kv.second[m + z]];
+                        hslice[nslice + z] = (int32_t)(it.first - items[j].first);
+                        hslice[nslice + G.nslices + z] = (int32_t)it.count;
+                    }
+                    nslice += 2 * (size_t)G.nslices;
+                    G.factor_begin = H.nfactors;
+                    H.nfactors += (long long)G.nslices * G.quads * G.nchunks;
+                    G.task_begin = H.ntasks;
+                    H.ntasks += (long long)G.ctx.nl * G.nchunks * G.parts;
+                    ++H.nsegs;
+                    m = e;
+                }
+                int rc = hist_prepare(H, p0.nbins, p0.pair_warps);
+                if (rc) return rc;
+                W.launches.push_back(Lc);
+                continue;
+            }
+            Lc.fn = pick_batch_pairs(p0.nbins);
+            Lc.warps = p0.pair_warps ? p0.pair_warps : pair_block_warps((p0.nbins + 1) / 2, false);
+            if (!Lc.fn) return sss_set_error(SSS_ERR_INVALID, "sss_batch_plan: nbins out of range");
+            for (size_t j : kv.second) {
+                const Item& it = items[j];
+                const sss_tof_problem& p = problems[it.prob];
+                PairItem& P = hpair[pk++];
+                P.ctx = context(j);
                 P.npts = (int)it.count;
                 P.nchunks = pair_chunks(p.nru, p.ndu);
                 P.task_begin = Lc.ntasks;
-                Lc.ntasks += (long long)C.nl * P.nchunks;
+                Lc.ntasks += (long long)P.ctx.nl * P.nchunks;
             }
             int rc = prepare_batch_pairs(Lc.fn, Lc.nbins, Lc.warps, Lc.ntasks, &Lc.blocks);
             if (rc) return rc;
@@ -480,6 +606,19 @@ int plan_items(const sss_tof_problem* problems, int32_t n, float* const* outs,
             cudaMemcpyAsync(dpair, hpair.data(), sizeof(PairItem) * hpair.size(), cudaMemcpyHostToDevice,
                             st) != cudaSuccess)
             return sss_set_error(SSS_ERR_CUDA, "sss_batch_plan: descriptor upload failed");
+        if (nseg && (cudaMemcpyAsync(dseg, hseg.data(), sizeof(HistSeg) * nseg, cudaMemcpyHostToDevice, st) !=
+                         cudaSuccess ||
+                     cudaMemcpyAsync(dslice, hslice.data(), sizeof(int32_t) * nslice, cudaMemcpyHostToDevice, st) !=
+                         cudaSuccess))
+            return sss_set_error(SSS_ERR_CUDA, "sss_batch_plan: descriptor upload failed");
+        std::map<TofClass, bool> filled;
+        for (const Item& it : items) {
+            const sss_tof_problem& p = problems[it.prob];
+            if (!rows_off.count(tof_class(p)) || filled[tof_class(p)]) continue;
+            int rc = hist_fill_rows(p, (float*)(ws + rows_off[tof_class(p)]), st);
+            if (rc) return rc;
+            filled[tof_class(p)] = true;
+        }
         if (cudaStreamSynchronize(st) != cudaSuccess)
             return sss_set_error(SSS_ERR_CUDA, "sss_batch_plan: %s", cudaGetErrorString(cudaGetLastError()));
     }
@@ -517,7 +656,14 @@ extern "C" int sss_batch_run_waves(const sss_batch* B, int32_t first, int32_t co
         batch_leg_kernel<<<(unsigned)((W.threads + lt - 1) / lt), lt, 0, st>>>(W.legs, W.nlegs, W.threads);
         int rc = sss_check_launch("batch_leg_kernel");
         if (rc) return rc;
+        for (const auto& c : W.clear)
+            if (cudaMemsetAsync(c.first, 0, c.second, st) != cudaSuccess)
+                return sss_set_error(SSS_ERR_CUDA, "sss_batch_run: memset failed");
         for (const auto& L : W.launches) {
+            if (L.hist) {
+                if ((rc = hist_enqueue(L.hl, st))) return rc;
+                continue;
+            }
             L.fn<<<(unsigned)L.blocks, L.warps * 32, pair_smem_bytes(L.nbins),
                    st>>>(
                 L.items, L.nitems, L.ntasks, L.T, L.tof, L.counter, B->status);
@@ -538,7 +684,10 @@ extern "C" int sss_batch_info(const sss_batch* B, int64_t* info)
 {
     if (!B || !info) return sss_set_error(SSS_ERR_INVALID, "sss_batch_info: bad argument");
     int64_t launches = 0;
-    for (const auto& W : B->waves) launches += 1 + (int64_t)W.launches.size();
+    for (const auto& W : B->waves) {
+        launches += 1 + (int64_t)W.launches.size();
+        for (const auto& L : W.launches) launches += L.hist && !L.hl.unit;  // factors, then the histogram
+    }
     info[0] = (int64_t)B->waves.size();
     info[1] = launches;
     info[2] = B->units;

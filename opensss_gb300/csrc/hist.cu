@@ -1,0 +1,565 @@
+// The pair stage as sums per (detector pair, TOF offset) (see hist.cuh):
+// kernels and launches.
+#include <algorithm>
+
+#include "hist.cuh"
+
+namespace sss {
+namespace {
+
+constexpr int kMaxScale = 120;
+
+// Block state beside the histogram.
+struct HistCtl {
+    HistSeg seg;
+    long long task;
+    int scale[32];  // the column's terms are in units of 2^-scale
+    int next;       // the task's next 8 points
+};
+
+constexpr int kHistCtlBytes = (sizeof(HistCtl) + 15) / 16 * 16;
+constexpr int kHistVoxBytes = kHistWarps * 32 * (int)sizeof(float2);
+
+// 2^e for |e| <= 126.
+__device__ __forceinline__ float pow2i(int e) { return __int_as_float((e + 127) << 23); }
+
+// The smallest k with x <= 2^k (x normal; -127 for zero).
+__device__ __forceinline__ int ceil_log2(float x)
+{
+    const int b = __float_as_int(x);
+    return ((b >> 23) & 0xFF) - 127 + ((b & 0x7FFFFF) ? 1 : 0);
+}
+
+__device__ __forceinline__ void red_add(uint32_t addr, int v)
+{
+    // volatile keeps its place among the barriers; no memory clobber, so that loaded values stay in registers
+    asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(addr), "r"(v));
+}
+
+// A collected bound of offsets, clamped so that its floor stays exact and beyond the table.
+__device__ __forceinline__ int floor_clamped(float x) { return floor_small(fminf(fmaxf(x, -1.0e6f), 1.0e6f)); }
+
+// The launch's run that holds task `task` (begin: prefix of tasks).
+template <long long HistSeg::*begin>
+__device__ __forceinline__ int find_seg(const HistSeg* segs, int n, long long task)
+{
+    int a = 0, b = n - 1;
+    while (a < b) {
+        const int mid = (a + b + 1) >> 1;
+        if (segs[mid].*begin <= task) a = mid;
+        else b = mid - 1;
+    }
+    return a;
+}
+
+// Partner entry q of walking leg lw (legs are crystal-major): legs 0..nl-1 (lw
+// leads the pair unless its crystal is the larger, :469), then one more entry
+// per other ring for the same crystal in the opposite role (both orders are
+// distinct pairs).  lp == lw: no pair.
+struct Partner {
+    int lp;
+    bool w_first;
+};
+__device__ __forceinline__ Partner partner_of(int q, int lw, int nl, int nru)
+{
+    if (q < nl) return {q, q / nru >= lw / nru};
+    if (q < nl + nru) return {lw / nru * nru + (q - nl), false};
+    return {lw, true};
+}
+// The walked leg's samples enter the TOF offset with this sign (:520 for leg 1, :526 for leg 2).
+__device__ __forceinline__ float walk_sign(bool w_first) { return w_first ? -1.f : 1.f; }
+
+// The pairs' factors: a warp takes one slice, kFactorLegs walking legs and 32
+// partner entries.  A partner's record serves all its walking legs, whose
+// chains of dependent operations overlap; the walking legs' records are read
+// by the block's other warps too (they take neighbouring chunks).  Bound by
+// instruction issue (about 90 per point, walking leg and 32 pairs).
+template <bool BATCH, bool UNIT>
+__global__ void __launch_bounds__(kFactorWarps * 32, 3) factor_kernel(const __grid_constant__ HistLaunch P)
+{
+    // a single problem's energy table, in shared memory; a batch's problems have their own
+    __shared__ float2 energy[BATCH ? 1 : kRowEnd - kRowFirst];
+    const int lane = threadIdx.x & 31;
+    const long long task = (long long)blockIdx.x * kFactorWarps + (threadIdx.x >> 5);
+    if (!BATCH) {
+        for (int i = threadIdx.x; i < kRowEnd - kRowFirst; i += blockDim.x)
+            energy[i] = make_float2(__ldg(P.one.ctx.eff + kRowFirst + i), __ldg(P.one.ctx.ratio + kRowFirst + i));
+        __syncthreads();
+    }
+    if (task >= P.nfactors) return;
+    const HistSeg& G = BATCH ? P.segs[find_seg<&HistSeg::factor_begin>(P.segs, P.nsegs, task)] : P.one;
+    const PairCtx& C = G.ctx;
+    const long long rem = task - G.factor_begin;
+    const int chunk = (int)(rem % G.nchunks), quad = (int)(rem / G.nchunks % G.quads);
+    const int slice = (int)(rem / G.nchunks / G.quads);
+    const int s0 = BATCH ? G.first[slice] : P.first[slice], n = BATCH ? G.count[slice] : P.count[slice];
+    const int nl = C.nl, Q = 32 * G.nchunks, q = chunk * 32 + lane;
+    const int lw0 = quad * kFactorLegs, legs = min(kFactorLegs, nl - lw0);
+    const bool mixed = chunk * 32 + 31 >= nl;  // partners that depend on the walking leg
+    const float inv_c = (float)(1.0 / kLightCmPerPs);
+    float cn[kFactorLegs], cs[kFactorLegs], sign_c[kFactorLegs];
+    float lo[kFactorLegs], hi[kFactorLegs], at_lo[kFactorLegs], at_hi[kFactorLegs];  // offsets, and the terms' size there
+    int lp[kFactorLegs];
+    unsigned word[kFactorLegs];
+#pragma unroll
+    for (int w = 0; w < kFactorLegs; ++w) {
+        const Partner pr = partner_of(q, lw0 + w, nl, C.nru);
+        lp[w] = w < legs ? pr.lp : lw0 + w;
+        sign_c[w] = walk_sign(pr.w_first) * inv_c;
+        cn[w] = cs[w] = 0.f;
+        lo[w] = INFINITY;
+        hi[w] = -INFINITY;
+        at_lo[w] = at_hi[w] = 0.f;
+        word[w] = 0;
+    }
+    const auto table = [&] {
+        if constexpr (BATCH) return GlobalEnergyTable{C.eff, C.ratio};
+        else return SharedEnergyTable{energy};
+    }();
+    bool energy_bad = false, nonfinite = false;
+    unsigned pairs = 0;
+    const float4* gA = C.legA + (long long)s0 * nl;  // the point's records
+    const float4* gB = C.legB + (long long)s0 * nl;
+    const float4* gD = C.legD + (long long)s0 * nl + lw0;
+    float* gC = G.f.c + ((long long)s0 * nl + lw0) * Q + q;
+    const long long c_step = (long long)nl * Q;
+    const int qa = min(q, nl - 1);
+    for (int s = s0; s < s0 + n; ++s) {
+        float4 Ap = __ldg(gA + qa), Bp = __ldg(gB + qa);
+#pragma unroll
+        for (int w = 0; w < kFactorLegs; ++w) {
+            if (w >= legs) break;
+            const float4 Aw = __ldg(gA + lw0 + w), Bw = __ldg(gB + lw0 + w);
+            if (mixed) {
+                Ap = __ldg(gA + lp[w]);
+                Bp = __ldg(gB + lp[w]);
+            }
+            const bool ok = lp[w] != lw0 + w && Aw.z != INFINITY && Ap.z != INFINITY && !(Aw.y == 0.f && Ap.y == 0.f);
+            float c = 0.f;
+            if (ok)
+                pairs += pair_term(C, table, s, Aw, Bw, Ap, Bp, (long long)s * nl, lw0 + w, lp[w], c, cn[w], energy_bad);
+            if (UNIT) {
+                cs[w] = fmaf(c, Aw.y, cs[w]);
+            } else {
+                const float4 Dw = __ldg(gD + w);
+                if (c != 0.f) {
+                    const float a = c * Dw.x;
+                    if (!isfinite(a)) {
+                        nonfinite = true;
+                        c = 0.f;
+                    } else {
+                        cs[w] += fabsf(a);
+                        // TOF offset index: floor(2((sv1-sv2)/2 -/+ r)/c + 0.5) + 4000 (:520, :526)
+                        const float u = fmaf(-sign_c[w], Aw.x - Ap.x, 4000.5f);
+                        const float sigma = sign_c[w] < 0.f ? -1.f : 1.f;
+                        const float xa = fmaf(sigma, Dw.y, u), xb = fmaf(sigma, Dw.z, u);
+                        const float x0 = fminf(xa, xb), x1 = fmaxf(xa, xb);
+                        if (x0 < lo[w]) at_lo[w] = fabsf(a);
+                        if (x1 > hi[w]) at_hi[w] = fabsf(a);
+                        lo[w] = fminf(lo[w], x0);
+                        hi[w] = fmaxf(hi[w], x1);
+                    }
+                }
+                __stcs(gC + w * Q, c);
+                if (__any_sync(0xffffffffu, c != 0.f)) word[w] |= 1u << (s & 31);
+            }
+        }
+        if (!UNIT && ((s & 31) == 31 || s == s0 + n - 1)) {  // this point ends a word
+#pragma unroll
+            for (int w = 0; w < kFactorLegs; ++w) {
+                if (lane == 0 && word[w])
+                    atomicOr(G.f.active + ((long long)(lw0 + w) * G.nchunks + chunk) * G.words + (s >> 5), word[w]);
+                word[w] = 0;
+            }
+        }
+        gA += nl;
+        gB += nl;
+        gD += nl;
+        gC += c_step;
+    }
+#pragma unroll
+    for (int w = 0; w < kFactorLegs; ++w) {
+        const int lw = lw0 + w;
+        if (w >= legs) break;
+        const float inv = cn[w] > 0.f ? 1.0f / cn[w] : 0.f;
+        const long long at = (long long)lw * Q + q;
+        if (UNIT) {
+            const float v = cs[w] * inv;
+            if (lp[w] != lw && v != 0.f) {
+                nonfinite |= !isfinite(v);
+                atomicAdd(C.out + (sign_c[w] < 0.f ? (long long)lw * nl + lp[w] : (long long)lp[w] * nl + lw), v);
+            }
+        } else {
+            G.f.inv[(long long)slice * nl * Q + at] = inv;
+            if (lo[w] <= hi[w]) {
+                atomicAdd(G.f.total + at, cs[w] * inv);
+                auto end = [&](int offset, float size) {
+                    return (unsigned long long)(unsigned)(kOffsetBias + offset) << 32 |
+                           (unsigned)__float_as_int(size * inv);
+                };
+                atomicMax(G.f.nlo + at, end(-floor_clamped(lo[w]), at_lo[w]));
+                atomicMax(G.f.nhi + at, end(floor_clamped(hi[w]), at_hi[w]));
+            }
+        }
+    }
+    finish_pairs(lane, false, energy_bad, nonfinite, 0, pairs, P.status, P.work);
+}
+
+// Multiplies the histogram's rows rlo..rhi by the TOF table and adds the
+// result to the output; clears the rows.  base: offset of row 0.
+__device__ void flush_rows(HistCtl& S, const HistSeg& G, int* hist, int rlo, int rhi, int base, float* partial,
+                           int warp, int warps, int lane, int lw, int lp, float sigma, bool& nonfinite)
+{
+    const bool lane_ok = lp != lw;
+    const int l1 = sigma < 0.f ? lw : lp, l2 = sigma < 0.f ? lp : lw;
+    const PairCtx& C = G.ctx;
+    const int stride = G.stride, nbins = C.nbins;
+    for (int bc = 0; bc < nbins; bc += kHistBinChunk) {
+        float acc[kHistBinChunk];
+#pragma unroll
+        for (int k = 0; k < kHistBinChunk; ++k) acc[k] = 0.f;
+        const bool last = bc + kHistBinChunk >= nbins;
+        for (int r = rlo + warp; r <= rhi; r += warps) {
+            const int v = hist[r * 32 + lane];
+            if (!__any_sync(0xffffffffu, v != 0)) continue;
+            if (last) hist[r * 32 + lane] = 0;
+            const int t = wrap_offset(base + r);  // numpy's negative index (:521, :527)
+            const float4* row = reinterpret_cast<const float4*>(G.rows + (long long)t * stride + bc);
+            const float f = (float)v;
+#pragma unroll
+            for (int k = 0; k < kHistBinChunk / 4; ++k) {
+                if (bc + 4 * k < stride) {
+                    const float4 w = __ldg(row + k);
+                    acc[4 * k] = fmaf(f, w.x, acc[4 * k]);
+                    acc[4 * k + 1] = fmaf(f, w.y, acc[4 * k + 1]);
+                    acc[4 * k + 2] = fmaf(f, w.z, acc[4 * k + 2]);
+                    acc[4 * k + 3] = fmaf(f, w.w, acc[4 * k + 3]);
+                }
+            }
+        }
+        const int nb = min(kHistBinChunk, nbins - bc);
+#pragma unroll
+        for (int k = 0; k < kHistBinChunk; ++k)
+            if (k < nb) partial[(k * warps + warp) * 32 + lane] = acc[k];
+        __syncthreads();
+        for (int b = warp; b < nb; b += warps) {  // one warp a bin: sums the warps' partials
+            float s = 0.f;
+            for (int w = 0; w < warps; ++w) s += partial[(b * warps + w) * 32 + lane];
+            const float v = s * pow2i(-S.scale[lane]);
+            if (lane_ok && v != 0.f) {
+                nonfinite |= !isfinite(v);
+                atomicAdd(C.out + (long long)(bc + b) * C.nl * C.nl + (long long)l1 * C.nl + l2, v);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Every active pair's voxels into the block's histogram, which is then
+// multiplied by the TOF table.  Bound by instruction issue: about 7 a voxel of
+// the walking leg and 32 pairs (offset, fixed-point term, shared add), about 60
+// a scatter point; shared memory carries under 2 wavefronts a voxel.
+template <bool BATCH>
+__global__ void __launch_bounds__(kHistWarps * 32, 1) hist_kernel(const __grid_constant__ HistLaunch P)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    HistCtl& S = *reinterpret_cast<HistCtl*>(smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    float2* vbuf = reinterpret_cast<float2*>(smem + kHistCtlBytes) + warp * 32;
+    int* hist = reinterpret_cast<int*>(smem + kHistCtlBytes + kHistVoxBytes);
+    const uint32_t hist_lane = (uint32_t)__cvta_generic_to_shared(hist) + 4u * lane;
+    float* const partial = P.partial + (long long)blockIdx.x * (kHistWarps * kHistBinChunk * 32);
+    const int R = P.rows;
+    for (int i = threadIdx.x; i < R * 32; i += blockDim.x) hist[i] = 0;
+    const float inv_c = (float)(1.0 / kLightCmPerPs);
+    int cur = -1;
+    bool tof_bad = false, nonfinite = false;
+    unsigned long long walked = 0;
+
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) S.task = atomicAdd(P.counter, 1u);
+        __syncthreads();
+        const long long task = S.task;
+        if (task >= P.ntasks) break;
+        if (BATCH) {
+            const int a = find_seg<&HistSeg::task_begin>(P.segs, P.nsegs, task);
+            if (a != cur) {  // the same run for every thread
+                static_assert(sizeof(HistSeg) % 4 == 0, "copied as words");
+                const int* src = reinterpret_cast<const int*>(P.segs + a);
+                int* dst = reinterpret_cast<int*>(&S.seg);
+                for (int i = threadIdx.x; i < (int)(sizeof(HistSeg) / 4); i += blockDim.x) dst[i] = __ldg(src + i);
+                cur = a;
+                __syncthreads();
+            }
+        }
+        const HistSeg& G = BATCH ? S.seg : P.one;  // a single problem's constants come from the parameter bank
+        const int* const first = BATCH ? S.seg.first : P.first;
+        const PairCtx& C = G.ctx;
+        const int nl = C.nl, Q = 32 * G.nchunks;
+        int lw, chunk, w_begin, w_end;
+        {
+            const long long rem = task - G.task_begin, per = (long long)G.nchunks * G.parts;
+            lw = (int)(rem / per);
+            chunk = (int)(rem % per) / G.parts;
+            const int part = (int)(rem % per) % G.parts;
+            w_begin = (int)((long long)part * G.words / G.parts);  // words of 32 points
+            w_end = (int)((long long)(part + 1) * G.words / G.parts);
+        }
+        const int q = chunk * 32 + lane;
+        const Partner pr = partner_of(q, lw, nl, C.nru);
+        const float sigma = walk_sign(pr.w_first), sign_c = sigma * inv_c;
+        // the columns' scales and the offsets they span
+        const long long at = (long long)lw * Q + q;
+        const float total = __ldg(G.f.total + at);
+        const unsigned long long nlo = __ldg(G.f.nlo + at), nhi = __ldg(G.f.nhi + at);
+        const int t_lo = nlo ? kOffsetBias - (int)(nlo >> 32) : INT_MAX, t_hi = nhi ? (int)(nhi >> 32) - kOffsetBias : INT_MIN;
+        int glo = __reduce_min_sync(0xffffffffu, t_lo), ghi = __reduce_max_sync(0xffffffffu, t_hi);
+        if (glo > ghi) continue;  // no terms
+        const bool beyond = glo < -kTofEntries || ghi > kTofEntries - 1;
+        tof_bad |= beyond;  // the reference's IndexError; the offsets beyond the table add nothing
+        glo = max(glo, -kTofEntries);
+        ghi = min(ghi, kTofEntries - 1);
+        int scale = 0;
+        if (total > 0.f) {  // the terms' roundings stay within 2^31 - 2^30.9
+            scale = isfinite(total) ? max(-kMaxScale, min(kMaxScale, 31 - ceil_log2(total))) : -kMaxScale;
+            if (total * pow2i(scale) > 2.0e9f) --scale;
+        }
+        if (warp == 0) S.scale[lane] = scale;
+        const float unit = pow2i(scale);
+        const int cap2 = C.cap - 2;
+        const float* const gC = G.f.c + at;
+        const float* const gI = G.f.inv + at;
+        const float4 *const gAw = C.legA + lw, *const gAp = C.legA + pr.lp, *const gD = C.legD + lw;
+        const float2* const gVl = C.vox + (long long)lw * C.cap + lane;
+        const unsigned c_step = (unsigned)nl * Q, v_step = (unsigned)nl * C.cap;  // below 2^32 (hist_form)
+        auto at_point = [](auto* base, int s, unsigned step) { return base + (unsigned long long)(unsigned)s * step; };
+        const unsigned* const active = G.f.active + ((long long)lw * G.nchunks + chunk) * G.words;
+
+        for (int base = glo; base <= ghi; base += R) {  // windows of R offsets
+            const int top = min(base + R - 1, ghi);
+            const bool check = beyond || top - base < ghi - glo;  // terms outside the window are left out
+            const uint32_t addr0 = hist_lane - (0x4B400000u + (uint32_t)base) * 128u;
+            if (threadIdx.x == 0) S.next = 4 * w_begin;
+            __syncthreads();
+            int slice = 0, slice_end = G.nslices > 1 ? first[1] : INT_MAX;
+            float inv = __ldg(gI);
+            for (;;) {
+                int wi = 0;
+                if (lane == 0) wi = atomicAdd(&S.next, 1);
+                wi = __shfl_sync(0xffffffffu, wi, 0);
+                if (wi >= 4 * w_end) break;
+                unsigned bits = __ldg(active + (wi >> 2)) >> (8 * (wi & 3)) & 0xFFu;  // 8 points
+                if (!bits) continue;
+                // the next point's factors, list record and first 32 voxels are loaded one point ahead
+                int s = wi * 8 + __ffs((int)bits) - 1;
+                bits &= bits - 1;
+                float c0, sp;
+                float4 D;
+                float sw;
+                float2 v0 = make_float2(0.f, 0.f);
+                auto load = [&]() {
+                    c0 = __ldcs(at_point(gC, s, c_step));
+                    D = __ldg(at_point(gD, s, nl));
+                    sp = __ldg(&at_point(gAp, s, nl)->x);
+                    sw = __ldg(&at_point(gAw, s, nl)->x);
+                    if (lane < cap2) v0 = __ldg(at_point(gVl, s, v_step));
+                };
+                load();
+                for (bool more = true; more;) {
+                    const int s1 = s;
+                    const float c1 = c0, d1 = sw - sp;
+                    const float4 D1 = D;
+                    const float2 v1 = v0;
+                    more = bits != 0;
+                    if (more) {
+                        s = wi * 8 + __ffs((int)bits) - 1;
+                        bits &= bits - 1;
+                        load();
+                    }
+                    if (s1 >= slice_end) {  // points come in ascending order to every warp
+                        do {
+                            ++slice;
+                            slice_end = slice + 1 < G.nslices ? first[slice + 1] : INT_MAX;
+                        } while (s1 >= slice_end);
+                        inv = __ldg(at_point(gI, slice, c_step));
+                    }
+                    const float c = c1 * inv * unit;
+                    // TOF offset index: floor(2((sv1-sv2)/2 -/+ r)/c + 0.5) + 4000 (:520, :526)
+                    const float u = fmaf(-sign_c, d1, 4000.5f);
+                    const int nw = min(__float_as_int(D1.w), cap2);
+                    // terms that all round to 0 on the column's grid are not walked
+                    const bool act = fabsf(c) * D1.x >= 0.5f;
+                    if (!__any_sync(0xffffffffu, act)) continue;
+                    if (act) walked += nw;
+                    for (int k0 = 0; k0 < nw; k0 += 32) {
+                        const int jn = min(32, nw - k0);
+                        float2 v = v1;
+                        if (k0 && lane < jn) v = __ldg(at_point(gVl, s1, v_step) + k0);
+                        if (lane >= jn) v = make_float2(0.f, D1.y);
+                        __syncwarp();
+                        vbuf[lane] = v;
+                        __syncwarp();
+                        if (act) {
+                            const float4* v4 = reinterpret_cast<const float4*>(vbuf);
+                            if (!check) {
+                                auto add = [&](float a, float rho) {
+                                    const float x = fmaf(sigma, rho, u);
+                                    const uint32_t t = __float_as_uint(__fadd_rd(x, 12582912.0f));
+                                    red_add(t * 128u + addr0, __float2int_rn(c * a));
+                                };
+                                for (int m = 0; m < jn; m += 4) {
+                                    const float4 a = v4[m / 2], b = v4[m / 2 + 1];
+                                    add(a.x, a.y);
+                                    add(a.z, a.w);
+                                    add(b.x, b.y);
+                                    add(b.z, b.w);
+                                }
+                            } else {
+                                for (int m = 0; m < jn; ++m) {
+                                    const int t = floor_small(fmaf(sigma, vbuf[m].y, u)) - base;
+                                    if ((unsigned)t <= (unsigned)(top - base))
+                                        red_add(hist_lane + (uint32_t)t * 128u, __float2int_rn(c * vbuf[m].x));
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            flush_rows(S, G, hist, 0, top - base, base, partial, warp, warps, lane, lw, pr.lp, sigma, nonfinite);
+        }
+    }
+    finish_pairs(lane, tof_bad, false, nonfinite, walked, 0, P.status, P.work);
+}
+
+// A bin that only terms far below a column's total reach (they round to 0 on
+// its grid) comes out of the histogram as exactly 0, where the reference has a
+// tiny positive value.  Such cells get the size of the terms at the column's
+// smallest and largest offset times the weight there: what the bins beyond the
+// offsets' range, the only ones concerned, are made of.  One thread an ordered
+// pair (lw leading); the pair's other column is that of the partner's walk.
+template <bool BATCH>
+__global__ void __launch_bounds__(256) fill_zero_kernel(const __grid_constant__ HistLaunch P)
+{
+    const HistSeg& G = BATCH ? P.segs[blockIdx.z] : P.one;
+    const PairCtx& C = G.ctx;
+    const int nl = C.nl, Q = 32 * G.nchunks, lp = blockIdx.x * blockDim.x + threadIdx.x, lw = blockIdx.y;
+    if (lp >= nl || lw >= nl || lp == lw) return;
+    const int dw = lw / C.nru, dp = lp / C.nru;
+    if (dp < dw) return;
+    // the partner's walk: entry lw, or the same crystal's second entry
+    const long long mine = (long long)lw * Q + lp, other = (long long)lp * Q + (dp == dw ? nl + lw - dw * C.nru : lw);
+    unsigned long long end[4] = {G.f.nlo[mine], G.f.nhi[mine], G.f.nlo[other], G.f.nhi[other]};
+    const float* row[4];
+    float size[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int off = end[k] ? (int)(end[k] >> 32) - kOffsetBias : 0;
+        const int t = wrap_offset(k & 1 ? off : -off);
+        const bool in = end[k] && (unsigned)t < (unsigned)kTofEntries;
+        size[k] = in ? __int_as_float((int)(unsigned)end[k]) : 0.f;
+        row[k] = G.rows + (long long)(in ? t : 0) * G.stride;
+    }
+    if (!end[0] && !end[2]) return;
+    float* o = C.out + (long long)lw * nl + lp;
+    for (int b = 0; b < C.nbins; ++b, o += (long long)nl * nl) {
+        if (*o != 0.f) continue;
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v = fmaxf(v, size[k] * __ldg(row[k] + b));
+        if (v != 0.f) *o = v;
+    }
+}
+
+// TOF weights of every offset, from the (log2 largest weight, its bin) table:
+// w_b = 2^(Y - d (beta + gamma d)), d = n - b (the Gaussian's exact ratio
+// between bins); the exponent in FP64.
+__global__ void __launch_bounds__(256) tof_rows_kernel(const float* __restrict__ log2w, int nbins, int stride, double s0,
+                                                       double w, double kappa, float* __restrict__ rows)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kTofEntries * stride) return;
+    const int t = i / stride, b = i % stride;
+    float v = 0.f;
+    if (b < nbins) {
+        const double Y = log2w[2 * t], n = log2w[2 * t + 1];
+        const double d = n - b, beta = 2.0 * kappa * w * ((t - kTimeRange) - (s0 + n * w));
+        const double e = Y - d * (beta + kappa * w * w * d);
+        if (e > -200.0) {
+            const double k = floor(e);
+            v = ldexpf(exp2f((float)(e - k)), (int)k);
+        }
+    }
+    rows[i] = v;
+}
+
+}  // namespace
+
+int hist_fill_rows(const sss_tof_problem& p, float* rows, cudaStream_t st)
+{
+    const int stride = hist_stride(p.nbins), n = kTofEntries * stride;
+    const double w = p.tof_bin_width, kappa = 4.0 / (p.tof_resolution * p.tof_resolution);
+    tof_rows_kernel<<<(n + 255) / 256, 256, 0, st>>>(p.tof_log2w, p.nbins, stride, (1.0 - (p.nbins + 1) / 2.0) * w, w,
+                                                     kappa, rows);
+    return sss_check_launch("tof_rows_kernel");
+}
+
+namespace {
+
+using LaunchFn = void (*)(const HistLaunch);
+
+}  // namespace
+
+// A run with fewer (walking leg, chunk) tasks than four a multiprocessor is
+// split over its points too.
+void hist_shape(const sss_tof_problem& p, int nslices, int npts, HistSeg& G)
+{
+    const long long nl = (long long)p.nru * p.ndu;
+    G.stride = hist_stride(p.nbins);
+    G.nchunks = pair_chunks(p.nru, p.ndu);
+    G.quads = (int)((nl + kFactorLegs - 1) / kFactorLegs);
+    G.nslices = nslices;
+    G.npts = npts;
+    G.words = (npts + 31) / 32;
+    const long long tasks = std::max<long long>(1, nl * G.nchunks);
+    G.parts = (int)std::max<long long>(1, std::min<long long>(G.words, (4 * kHistBlocks + tasks - 1) / tasks));
+}
+
+// pair_warps (sss_tof_problem) is taken as a share of the full block, in units
+// of 1 / sss_pair_warps_max.
+int hist_prepare(HistLaunch& L, int nbins, int pair_warps)
+{
+    L.rows = L.smem = L.warps = L.blocks = 0;
+    if (L.unit) return SSS_OK;
+    int dev = 0, sms = 0, most = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const int bound = pair_block_warps((nbins + 1) / 2, false);
+    L.warps = pair_warps > 0 ? std::max(1, kHistWarps * pair_warps / bound) : kHistWarps;
+    L.rows = (most - kHistCtlBytes - kHistVoxBytes) / 128;
+    if (L.rows < 64) return sss_set_error(SSS_ERR_CUDA, "pair stage: %d bytes of shared memory a block", most);
+    L.smem = kHistCtlBytes + kHistVoxBytes + L.rows * 128;
+    const LaunchFn fn = L.segs ? hist_kernel<true> : hist_kernel<false>;
+    if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem) != cudaSuccess)
+        return sss_set_error(SSS_ERR_CUDA, "pair stage: %s", cudaGetErrorString(cudaGetLastError()));
+    L.blocks = (int)std::max<long long>(1, std::min<long long>(std::min(sms, kHistBlocks), L.ntasks));
+    return SSS_OK;
+}
+
+int hist_enqueue(const HistLaunch& L, cudaStream_t st)
+{
+    const LaunchFn factor = L.segs ? (L.unit ? factor_kernel<true, true> : factor_kernel<true, false>)
+                                   : (L.unit ? factor_kernel<false, true> : factor_kernel<false, false>);
+    factor<<<(unsigned)((L.nfactors + kFactorWarps - 1) / kFactorWarps), kFactorWarps * 32, 0, st>>>(L);
+    int rc = sss_check_launch("factor_kernel");
+    if (rc || L.unit) return rc;
+    (L.segs ? hist_kernel<true> : hist_kernel<false>)<<<(unsigned)L.blocks, L.warps * 32, L.smem, st>>>(L);
+    if ((rc = sss_check_launch("hist_kernel"))) return rc;
+    const dim3 grid((unsigned)((L.most_legs + 255) / 256), (unsigned)L.most_legs, (unsigned)(L.segs ? L.nsegs : 1));
+    (L.segs ? fill_zero_kernel<true> : fill_zero_kernel<false>)<<<grid, 256, 0, st>>>(L);
+    return sss_check_launch("fill_zero_kernel");
+}
+
+}  // namespace sss

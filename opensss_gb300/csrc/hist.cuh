@@ -1,0 +1,143 @@
+// The pair stage as sums per (detector pair, TOF offset).  Reference: bodySSS,
+// Python/openSSS/SingleScatterSimulationTOF.py:433-557.
+//
+// A pair's sum over scatter points and voxels, sum c a w_b(t), depends on the
+// voxel only through its integer TOF offset t (the reference's table column,
+// :520-528).  So the sums of c a per (detector pair, t) are collected first and
+// multiplied by the TOF table once at the end: sum_t H[t] w_b(t).  A voxel then
+// costs one shared-memory add whatever the number of bins, where evaluating
+// its weights costs two packed FP32 instructions and 8 bytes of shared-memory
+// table per two bins.  Two kernels:
+//
+//  * factor_kernel: c of every (scatter point, walking leg, partner leg) to
+//    memory, the slices' counts, and per (walking leg, partner leg) the bound of
+//    its terms' sum and the range of its offsets.  Two walking legs a warp
+//    share a partner leg's record.  With SSS_FLAG_UNIT_TOF (every weight 1)
+//    this is all: the sums of c times the walking leg's activity integral.
+//  * hist_kernel: one block = one walking leg and 32 partner legs (lane =
+//    partner), all its warps on different scatter points.  H is [offset][lane],
+//    so the lanes' adds never share a bank whatever their offsets are, and it
+//    fills the multiprocessor's shared memory (about 1600 offsets; a 10 cm body
+//    needs up to 1560, wider ones take the offsets in windows).  The adds are
+//    32-bit integer atomics (fire and forget, one wavefront), which all warps
+//    of the block can make into one H: each column is in fixed point with a
+//    power-of-two scale that puts its terms' bound just below 2^31.  Rounding a
+//    term to that grid costs less than a float accumulation of the same terms
+//    does (they are added exactly after it).
+// Measured (whole TofSSS.run, direct evaluation -> this form): 13 bins, 768 legs,
+// 3,270 points 52.3 -> 30.0 ms; 33 bins, 855 legs, 5,372 points 268 -> 67.3 ms.
+// Relative error against FP64: 2.3e-6 -> 9.7e-7 and 4.1e-6 -> 9.8e-7.
+#pragma once
+
+#include <limits.h>
+
+#include "common.cuh"
+#include "pair.cuh"
+
+namespace sss {
+
+constexpr int kHistWarps = 32;     // warps of a histogram block (one block a multiprocessor)
+constexpr int kFactorWarps = 8;    // warps of a factor block
+constexpr int kFactorLegs = 2;     // walking legs of a factor warp
+constexpr int kHistBlocks = 152;   // most histogram blocks of a launch: the GPU's multiprocessors
+constexpr int kHistBinChunk = 16;  // bins multiplied out together at a flush
+constexpr int kMaxWaveSlices = 256;
+
+// What factor_kernel leaves for hist_kernel, per run of slices: Q = 32 nchunks
+// partner entries, words = ceil(points / 32).
+struct FactorOut {
+    float* c;            // [point][nl][Q]
+    float* inv;          // [slice][nl][Q] 1 / count
+    // zeroed before factor_kernel:
+    float* total;        // [nl][Q] bound of the sum of the terms' magnitudes
+    // kOffsetBias - smallest and + largest offset (high word; 0: no terms), with
+    // the size of that scatter point's terms (low word, float bits)
+    unsigned long long *nlo, *nhi;  // [nl][Q]
+    unsigned* active;    // [nl][nchunks][words] bit s % 32 of word s / 32: point s has an active pair
+};
+constexpr int kOffsetBias = 1 << 21;
+
+// One problem's run of whole z-slices.
+struct HistSeg {
+    PairCtx ctx;             // legs indexed from the run's first point
+    FactorOut f;
+    const float* rows;       // TOF weights [8001][stride], 0 past the last bin
+    int stride;              // bins rounded up to a multiple of 4
+    int nchunks;             // 32-partner chunks per walking leg
+    int quads;               // groups of kFactorLegs walking legs
+    int parts;               // tasks the run's points are split over
+    int nslices, npts, words;
+    const int32_t* first;    // [nslices] first point of each slice
+    const int32_t* count;    // [nslices] points of each slice
+    long long factor_begin;  // prefix over the launch's runs of nslices * quads * nchunks
+    long long task_begin;    // prefix over the launch's runs of nl * nchunks * parts
+};
+
+struct HistLaunch {
+    HistSeg one;             // the run of a single-problem launch; its slices are first, count below
+    int first[kMaxWaveSlices], count[kMaxWaveSlices];
+    const HistSeg* segs;     // device, nsegs runs of a batch, or null
+    int nsegs, most_legs;    // runs; most sampled legs of a run
+    int unit;                // SSS_FLAG_UNIT_TOF problems: no histogram
+    long long nfactors, ntasks;
+    unsigned int* counter;   // zeroed
+    unsigned long long* work;  // [0] voxels added per pair, [1] pairs evaluated; may be null
+    int32_t* status;
+    float* partial;          // per block: the flush's partial sums
+    int rows, smem, warps, blocks;  // set by hist_prepare
+};
+
+inline int hist_stride(int nbins) { return (nbins + 3) / 4 * 4; }
+inline size_t hist_rows_bytes(int nbins) { return sizeof(float) * kTofEntries * (size_t)hist_stride(nbins); }
+inline size_t hist_partial_bytes() { return sizeof(float) * kHistBlocks * kHistWarps * kHistBinChunk * 32; }
+
+// Bytes of a run's FactorOut: the part per point, per slice, and the zeroed part.
+struct FactorSize {
+    size_t c, inv, zeroed;
+};
+inline FactorSize factor_size(const sss_tof_problem& p, long long npts, long long nslices)
+{
+    const size_t nl = (size_t)p.nru * p.ndu, chunks = pair_chunks(p.nru, p.ndu), Q = 32 * chunks;
+    return {4 * (size_t)npts * nl * Q, 4 * (size_t)nslices * nl * Q,
+            20 * nl * Q + 4 * nl * chunks * (((size_t)npts + 31) / 32)};
+}
+inline FactorOut factor_out(const sss_tof_problem& p, char* c, char* inv, char* zeroed)
+{
+    const size_t n = (size_t)p.nru * p.ndu * 32 * pair_chunks(p.nru, p.ndu);
+    FactorOut f;
+    f.c = (float*)c;
+    f.inv = (float*)inv;
+    f.nlo = (unsigned long long*)zeroed;
+    f.nhi = f.nlo + n;
+    f.total = (float*)(f.nhi + n);
+    f.active = (unsigned*)(f.total + n);
+    return f;
+}
+
+// Most sampled legs of the histogram form: the factors take 4 nl^2 bytes a
+// point, 67 MB at this limit (the voxel lists about 6).
+constexpr long long kHistMaxLegs = 4096;
+
+// Whether a problem's pair stage has the histogram; unit TOF weights take
+// factor_kernel alone.  The other forms: one TOF bin of varying weight, and the
+// precision launch (which also serves problems of more legs).
+inline bool hist_lists(const sss_tof_problem& p)
+{
+    return !(p.flags & SSS_FLAG_KAHAN) && p.nbins > 1 && (long long)p.nru * p.ndu <= kHistMaxLegs;
+}
+inline bool hist_form(const sss_tof_problem& p)
+{
+    return hist_lists(p) || ((p.flags & SSS_FLAG_UNIT_TOF) && !(p.flags & SSS_FLAG_KAHAN));
+}
+inline bool compensated_form(const sss_tof_problem& p)
+{
+    return (p.flags & SSS_FLAG_KAHAN) || (p.nbins > 1 && !hist_lists(p));
+}
+
+// Defined in hist.cu.
+int hist_fill_rows(const sss_tof_problem& p, float* rows, cudaStream_t st);
+void hist_shape(const sss_tof_problem& p, int nslices, int npts, HistSeg& G);  // chunks, parts, words
+int hist_prepare(HistLaunch& L, int nbins, int pair_warps);  // launch shape, shared-memory opt-in
+int hist_enqueue(const HistLaunch& L, cudaStream_t st);      // the launches
+
+}  // namespace sss

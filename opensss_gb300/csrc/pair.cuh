@@ -80,6 +80,7 @@ struct PairCtx {
     const float4* legA;      // [point][nl]
     const float4* legB;
     const float4* legC;      // low floats of legB's unit vectors, and of legA's distance
+    const float4* legD;      // voxel-list sums, ranges and lengths (histogram launches), else null
     const float2* vox;       // [point][nl][cap]
     const float* vox_lo;     // [point][nl][cap] low floats of the samples (Kahan launches), else null
     float* out;              // [nbins][nl][nl]
@@ -393,6 +394,70 @@ __device__ __forceinline__ void accumulate_voxel(float2 (&acc)[NP], float ca, in
     }
 }
 
+// Rows of the energy tables a pair can take: 511 / (2 + q) lies in 170.3..511 keV.
+constexpr int kRowFirst = 336, kRowEnd = 1024;
+
+// (efficiency, attenuation ratio) of an energy row.
+struct GlobalEnergyTable {
+    const float* eff;
+    const float* ratio;
+    __device__ __forceinline__ float2 row(int r) const { return make_float2(__ldg(eff + r), __ldg(ratio + r)); }
+};
+struct SharedEnergyTable {
+    const float2* t;  // rows kRowFirst..kRowEnd-1
+    __device__ __forceinline__ float2 row(int r) const { return t[r - kRowFirst]; }
+};
+
+// The part of a detector pair's scatter term that does not depend on the
+// voxels: c, the factor of the walking leg's activity (0 where it has none),
+// and the pair's contribution to the slice's count.  Aw, Bw and Ap, Bp are the
+// leg records of the walking leg lw and the partner leg lp at point s; first is
+// the point's first record in legC (read only where the high floats do not
+// decide the energy row).
+// Returns whether the pair counts; everything here is symmetric in the two
+// legs but for the attenuation exponents.
+template <class Table>
+__device__ __forceinline__ bool pair_term(const PairCtx& C, const Table& tab, int s, float4 Aw, float4 Bw, float4 Ap,
+                                          float4 Bp, long long first, int lw, int lp, float& c, float& cnt,
+                                          bool& energy_bad)
+{
+    // cos of the angle between the legs = -cos(scatter angle) (:495, :498-499)
+    // and the scattered energy's row.  In FP32 from the legs' high floats
+    // the energy is within 3e-4 keV of the FP64 value, which decides the
+    // row except within 1e-3 keV of a rounding boundary (one pair in 500):
+    // there the float pairs decide it, and FP64 only within 1e-6 keV (about
+    // one pair in a million).
+    float qc = fmaf(Bw.x, Bp.x, fmaf(Bw.y, Bp.y, Bw.z * Bp.z));
+    qc = fminf(1.f, fmaxf(-1.f, qc));
+    const float e = __fdividef(511.0f, 2.0f + qc);
+    const float eh = e + 0.5f;
+    const float m = __fadd_rd(eh, 12582912.0f);  // floor(eh) in the mantissa
+    const float fr = eh - (m - 12582912.0f);
+    int row = 2 * (__float_as_int(m) - 0x4B400000) - 1;
+    if (fr < 1e-3f || fr > 1.0f - 1e-3f || fabsf(qc) > 1.0f - 1e-5f) {
+        row = energy_row_pair(Bw, C.legC[first + lw], Bp, C.legC[first + lp], qc);
+        if (row == -2) row = energy_row_fp64(C, s, lw % C.nru, lw / C.nru, lp % C.nru, lp / C.nru);
+        if (row < kRowFirst || row >= kRowEnd) {
+            energy_bad = true;
+            return false;
+        }
+    }
+    const float2 er = tab.row(row);
+    if (er.x == 0.f) return false;  // :508-509 skips before the count is added
+    // Klein-Nishina with cos(theta) = -qc (:239-258): Ratio = 1/den
+    const float den = fmaf(C.gamma_kn, 1.0f + qc, 1.0f);
+    const float ratio = __frcp_rn(den);
+    const float sin2 = fmaf(-qc, qc, 1.0f);
+    const float kn = ratio * ratio * (ratio + den - sin2);
+    // geometry (:533-536): (ds)^2 |cos a1||cos a2| / (4 pi sv1^2 sv2^2)
+    const float f = C.geo_c * (Aw.w * Ap.w) * (er.x * kn);
+    // this task's part: M1 * M2^r * AB1 or M2 * M1^r * AB2 (:540)
+    const float mw = ex2(-Aw.z), mpr = ex2(-er.y * Ap.z);
+    if (Aw.y != 0.f) c = f * mw * mpr;
+    cnt += (Aw.y != 0.f && Ap.y != 0.f) ? 2.f : 1.f;  // :485-488
+    return true;
+}
+
 // One task.  Every lane pairs lw with its own partner leg lp; the pair
 // (l1, l2) is ordered as the reference orders it (crystal of l1 < crystal of
 // l2, :469).  The task adds the part of the pair's TOF sum that runs over
@@ -459,46 +524,7 @@ __device__ __forceinline__ void walk_task(const PairCtx& C, const TofConst& T, i
         // everything below but the TOF offset's sign is symmetric in the two legs
         bool ok = lane_ok && Aw.z != INFINITY && Ap.z != INFINITY && !(Aw.y == 0.f && Ap.y == 0.f);
         float c = 0.f;
-        if (ok) {
-            // cos of the angle between the legs = -cos(scatter angle) (:495, :498-499)
-            // and the scattered energy's row.  In FP32 from the legs' high floats
-            // the energy is within 3e-4 keV of the FP64 value, which decides the
-            // row except within 1e-3 keV of a rounding boundary (one pair in 500):
-            // there the float pairs decide it, and FP64 only within 1e-6 keV (about
-            // one pair in a million).
-            float qc = fmaf(Bw.x, Bp.x, fmaf(Bw.y, Bp.y, Bw.z * Bp.z));
-            qc = fminf(1.f, fmaxf(-1.f, qc));
-            const float e = __fdividef(511.0f, 2.0f + qc);
-            const float eh = e + 0.5f;
-            const float fr = eh - floorf(eh);
-            int row;
-            if (fr < 1e-3f || fr > 1.0f - 1e-3f || fabsf(qc) > 1.0f - 1e-5f) {
-                row = energy_row_pair(Bw, C.legC[lo + lw], Bp, C.legC[lo + lp], qc);
-                if (row == -2) row = energy_row_fp64(C, s, rw, dw, rp, dp);
-            } else {
-                row = 2 * (int)floorf(eh) - 1;
-            }
-            if (row < 0 || row >= 2000) {
-                energy_bad = true;
-            } else {
-                const float effp = __ldg(C.eff + row);
-                if (effp != 0.f) {  // :508-509 skips before the count is added
-                    const float rr = __ldg(C.ratio + row);
-                    // Klein-Nishina with cos(theta) = -qc (:239-258): Ratio = 1/den
-                    const float den = fmaf(C.gamma_kn, 1.0f + qc, 1.0f);
-                    const float ratio = __frcp_rn(den);
-                    const float sin2 = fmaf(-qc, qc, 1.0f);
-                    const float kn = ratio * ratio * (ratio + den - sin2);
-                    // geometry (:533-536): (ds)^2 |cos a1||cos a2| / (4 pi sv1^2 sv2^2)
-                    const float f = C.geo_c * (Aw.w * Ap.w) * (effp * kn);
-                    // this task's part: M1 * M2^r * AB1 or M2 * M1^r * AB2 (:540)
-                    const float mw = ex2(-Aw.z), mpr = ex2(-rr * Ap.z);
-                    if (Aw.y != 0.f) c = f * mw * mpr;
-                    cnt += (Aw.y != 0.f && Ap.y != 0.f) ? 2.f : 1.f;  // :485-488
-                    npairs += 1;
-                }
-            }
-        }
+        if (ok && pair_term(C, GlobalEnergyTable{C.eff, C.ratio}, s, Aw, Bw, Ap, Bp, lo, lw, lp, c, cnt, energy_bad)) npairs += 1;
         // TOF offset index: floor(2((sv1-sv2)/2 -/+ r)/c + 0.5) + 4000 (:520, :526)
         float u = fmaf(-sigma * (Aw.x - Ap.x), inv_c, 4000.5f), ul = 0.f;
         if constexpr (KAHAN) {

@@ -1,17 +1,17 @@
-// The single-problem pair stage of sss_tof_run: kernel, launch and dispatch
-// over the bin count.  Shared by sss.cu (plain FP32 reduction over the
-// scatter points) and kahan.cu (Kahan-compensated reduction), which
+// The pair stage of sss_tof_run that evaluates the TOF weights voxel by
+// voxel: kernel, launch and dispatch over the bin count.  Shared by sss.cu (one
+// bin) and kahan.cu (the Kahan-compensated reduction, every bin count), which
 // instantiate disjoint sets of kernels so that the two compile in parallel.
+// The plain reduction of several bins is the histogram form (hist.cuh).
 #pragma once
 
 #include <algorithm>
 
 #include "common.cuh"
+#include "hist.cuh"
 #include "pair.cuh"
 
 namespace sss {
-
-constexpr int kMaxWaveSlices = 256;
 
 struct PairParams {
     PairCtx ctx;            // the problem (legs of the wave's first point at index 0)
@@ -80,9 +80,9 @@ int launch_pairs(const PairParams& P, cudaStream_t st)
     return sss_check_launch("pair_kernel");
 }
 
-template <bool KAHAN>
-int dispatch_pairs(const PairParams& P, cudaStream_t st)
+inline int dispatch_pairs_compensated(const PairParams& P, cudaStream_t st)
 {
+    constexpr bool KAHAN = true;
     if (P.ctx.nbins == 1) return launch_pairs<1, true, false, KAHAN>(P, st);
     const bool odd = P.ctx.nbins & 1;
     switch ((P.ctx.nbins + 1) / 2) {
@@ -99,8 +99,7 @@ int dispatch_pairs(const PairParams& P, cudaStream_t st)
     return sss_set_error(SSS_ERR_INVALID, "nbins out of range");
 }
 
-// Defined in sss.cu (plain) and kahan.cu (compensated).
-int dispatch_pairs_plain(const PairParams& P, cudaStream_t st);
+// Defined in kahan.cu.
 int dispatch_pairs_kahan(const PairParams& P, cudaStream_t st);
 
 }  // namespace sss

@@ -7,20 +7,22 @@
 //      Amanatides-Woo walk (bit-identical voxel sequence), FP32 integrals of
 //      mu and activity, incidence term, and the list of the leg's non-zero
 //      activity voxels (act*len, TOF sample offset), one list per leg.
-//   3. pair_kernel  — persistent warps pull (slice, walking leg, 32-partner
-//      chunk) tasks; each lane owns one detector pair, loops over the slice's
-//      scatter points, evaluates the Klein-Nishina x efficiency x attenuation
-//      factors once per pair, and for each voxel of the walking leg (staged in
-//      shared memory, read as broadcasts) adds the factored TOF weights
-//      [A r^b] G[n][b] of every bin from shared-memory tables; the slice
-//      numerator and count stay in registers and numerator/count is added to
-//      the output (per-slice normalisation, :555-557).
+//   3. the pair stage, each lane one detector pair, the Klein-Nishina x
+//      efficiency x attenuation factors once per pair and scatter point:
+//      several TOF bins: hist_kernel (hist.cuh), a histogram over the TOF
+//      offset multiplied by the TOF table at the end;
+//      unit TOF weights: the same kernel without the histogram;
+//      one bin of varying weight, and the precision launch: pair_kernel, where
+//      persistent warps pull (slice, walking leg, 32-partner chunk) tasks, the
+//      slice numerator and count stay in registers and numerator/count is added
+//      to the output (per-slice normalisation, :555-557).
 // Nothing per voxel or per pair reaches HBM except the leg lists themselves.
 #include <algorithm>
 #include <mutex>
 #include <vector>
 
 #include "common.cuh"
+#include "hist.cuh"
 #include "legs.cuh"
 #include "pair.cuh"
 #include "pair_launch.cuh"
@@ -247,7 +249,9 @@ struct StageTimer {
 thread_local StageTimer g_timer;
 
 struct WsLayout {
-    size_t legA, legB, legC, vox, vox_lo, counter, total;
+    size_t legA, legB, legC, legD, vox, vox_lo, counter, rows, partial, factor, inv, zeroed, total;
+    FactorSize sizes;
+    long long slices;  // most slices of a wave
 };
 
 WsLayout ws_layout(const sss_tof_problem& p, long long wave_points)
@@ -262,13 +266,31 @@ WsLayout ws_layout(const sss_tof_problem& p, long long wave_points)
     off = align_up(off + sizeof(float4) * wave_points * nl);
     w.legC = off;
     off = align_up(off + sizeof(float4) * wave_points * nl);
+    w.legD = off;
+    if (hist_lists(p)) off = align_up(off + sizeof(float4) * wave_points * nl);
     w.vox = off;  // no voxel lists when every TOF weight is 1
     const bool lists = !(p.flags & SSS_FLAG_UNIT_TOF);
     if (lists) off = align_up(off + sizeof(float2) * wave_points * cap * nl);
     w.vox_lo = off;  // the samples' low floats: the precision (Kahan) launch only
-    if (lists && (p.flags & SSS_FLAG_KAHAN)) off = align_up(off + sizeof(float) * wave_points * cap * nl);
+    if (lists && compensated_form(p)) off = align_up(off + sizeof(float) * wave_points * cap * nl);
     w.counter = off;
     off = align_up(off + 256);
+    w.slices = kMaxWaveSlices;
+    w.rows = w.partial = w.factor = w.inv = w.zeroed = off;
+    if (hist_lists(p)) {
+        w.slices = std::min<long long>(kMaxWaveSlices, lattice(p).lz);
+        w.sizes = factor_size(p, wave_points, w.slices);
+        auto take = [&](size_t bytes) {
+            const size_t at = off;
+            off = align_up(off + bytes);
+            return at;
+        };
+        w.rows = take(hist_rows_bytes(p.nbins));
+        w.partial = take(hist_partial_bytes());
+        w.factor = take(w.sizes.c);
+        w.inv = take(w.sizes.inv);
+        w.zeroed = take(w.sizes.zeroed);
+    }
     w.total = off;
     return w;
 }
@@ -303,9 +325,6 @@ int validate(const sss_tof_problem* p)
 }
 
 }  // namespace
-
-// The pair kernels of the plain reduction (the compensated ones are in kahan.cu).
-int sss::dispatch_pairs_plain(const PairParams& P, cudaStream_t st) { return dispatch_pairs<false>(P, st); }
 
 int sss_internal_validate(const sss_tof_problem* p) { return validate(p); }
 
@@ -423,8 +442,9 @@ extern "C" int sss_tof_run(const sss_tof_problem* p, const double* points, int64
     LP.legA = (float4*)(ws + w.legA);
     LP.legB = (float4*)(ws + w.legB);
     LP.legC = (float4*)(ws + w.legC);
+    LP.legD = hist_lists(*p) ? (float4*)(ws + w.legD) : nullptr;
     LP.vox = (p->flags & SSS_FLAG_UNIT_TOF) ? nullptr : (float2*)(ws + w.vox);
-    LP.vox_lo = (LP.vox && (p->flags & SSS_FLAG_KAHAN)) ? (float*)(ws + w.vox_lo) : nullptr;
+    LP.vox_lo = (LP.vox && compensated_form(*p)) ? (float*)(ws + w.vox_lo) : nullptr;
     LP.status = status;
 
     PairParams PP;
@@ -445,6 +465,7 @@ extern "C" int sss_tof_run(const sss_tof_problem* p, const double* points, int64
     C.legA = LP.legA;
     C.legB = LP.legB;
     C.legC = LP.legC;
+    C.legD = LP.legD;
     C.vox = LP.vox;
     C.vox_lo = LP.vox_lo;
     C.unit_tof = (p->flags & SSS_FLAG_UNIT_TOF) != 0;
@@ -458,6 +479,21 @@ extern "C" int sss_tof_run(const sss_tof_problem* p, const double* points, int64
     PP.status = status;
     PP.warps = p->pair_warps;
 
+    const bool hist = hist_form(*p);
+    HistLaunch HL = {};
+    if (hist) {
+        HL.unit = !hist_lists(*p);
+        HL.most_legs = (int)nl;
+        HL.counter = PP.counter;
+        HL.work = PP.work;
+        HL.status = status;
+        if (!HL.unit) {
+            HL.one.rows = (const float*)(ws + w.rows);
+            HL.partial = (float*)(ws + w.partial);
+            if ((rc = hist_fill_rows(*p, (float*)(ws + w.rows), st))) return rc;
+        }
+    }
+
     g_timer.clear();
     g_timer.work = PP.work;
     g_timer.nbins = p->nbins;
@@ -468,7 +504,7 @@ extern "C" int sss_tof_run(const sss_tof_problem* p, const double* points, int64
         long long npts = 0;
         int nsl = 0;
         PP.nslices = 0;
-        while (si < n_slices && nsl < kMaxWaveSlices && npts + slice_counts[si] <= wave_points) {
+        while (si < n_slices && nsl < w.slices && npts + slice_counts[si] <= wave_points) {
             if (slice_counts[si] > 0) {
                 PP.slice_first[PP.nslices] = (int)npts;
                 PP.slice_count[PP.nslices] = (int)slice_counts[si];
@@ -490,8 +526,24 @@ extern "C" int sss_tof_run(const sss_tof_problem* p, const double* points, int64
             PP.ctx.points = LP.points;
             cudaMemsetAsync(PP.counter, 0, sizeof(unsigned int), st);
             if (g_timer.on) cudaEventRecord(g_timer.get(), st);
-            if ((rc = (p->flags & SSS_FLAG_KAHAN) ? dispatch_pairs_kahan(PP, st) : dispatch_pairs_plain(PP, st)))
-                return rc;
+            if (hist) {
+                HL.one.ctx = PP.ctx;
+                hist_shape(*p, PP.nslices, (int)npts, HL.one);
+                std::copy(PP.slice_first, PP.slice_first + PP.nslices, HL.first);
+                std::copy(PP.slice_count, PP.slice_count + PP.nslices, HL.count);
+                HL.nfactors = (long long)PP.nslices * HL.one.quads * HL.one.nchunks;
+                HL.ntasks = nl * HL.one.nchunks * HL.one.parts;
+                if (!HL.unit) {
+                    HL.one.f = factor_out(*p, ws + w.factor, ws + w.inv, ws + w.zeroed);
+                    cudaMemsetAsync(ws + w.zeroed, 0, factor_size(*p, npts, PP.nslices).zeroed, st);
+                }
+                if ((rc = hist_prepare(HL, p->nbins, p->pair_warps))) return rc;
+                rc = hist_enqueue(HL, st);
+            } else {
+                rc = compensated_form(*p) ? dispatch_pairs_kahan(PP, st)
+                                          : launch_pairs<1, true, false, false>(PP, st);
+            }
+            if (rc) return rc;
             if (g_timer.on) cudaEventRecord(g_timer.get(), st);
             g_timer.launches += 2;
             g_timer.waves += 1;
