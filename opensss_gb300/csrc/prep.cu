@@ -10,6 +10,17 @@
 //      12 edge samples per side (recursive filter, pole sqrt(3) - 2);
 //   3. the coefficients sampled at x = (o + 0.5) in/out - 0.5 per axis;
 //   4. the result clipped to the [min, max] of the cropped input.
+// Steps 1 to 3 are linear and separable, and along one axis they are one short
+// filter per output sample, so an axis is done in one pass: every output sample
+// is a weighted sum of the input samples around it, the weights (Gaussian,
+// spline response and sampling multiplied out) formed once per axis in FP64.
+// The passes run from the last axis to the first and shrink the volume by each
+// axis' factor as they go, so the map is read once and nothing of its size is
+// written.  Measured, 400x400x280 map, 376x376x240 window to 75x75x48: eight
+// full-volume passes step by step 2.20 ms, this form 0.24 ms (0.18 of them the
+// pass over the map; its bytes at copy rate: 0.02 ms).
+// The step-by-step form remains for what the composed one does not cover (see
+// composed_fits).
 // Volumes are C-ordered float32 [n0][n1][n2].
 #include <math.h>
 
@@ -261,6 +272,316 @@ __global__ void zoom_kernel(const float* __restrict__ P, Dims dp, Dims din, floa
     }
 }
 
+// ---------------------------------------------------------------- composed form
+
+// Samples either side of a coefficient that its spline response takes: the
+// response falls as 0.268^distance, 3.6e-12 at this reach.  (The 12 repeated edge
+// samples and the mirror beyond them are then the same as repeating the edge
+// sample throughout.)
+constexpr int kReach = 20;
+constexpr int kTaps = 2 * kReach + 4;  // samples under an output sample's four coefficients
+constexpr int kGroup = 4;              // neighbouring output samples computed together
+constexpr int kLinePos = 512;          // samples of a line staged at once by line_axis_kernel
+constexpr int kLines = 32;             // lines of a line_axis_kernel block
+
+// One axis: n input samples, m output samples, Gaussian radius r (0: none).  A
+// group of kGroup output samples takes the input samples from start[g] on,
+// weight[g * span + u] being sample start[g] + u's weight in each of them.
+struct Axis {
+    int n, m, r, span, groups;
+    double sigma;
+    int* start;
+    float4* weight;
+};
+
+struct Axes {
+    Axis a[3];
+};
+
+__host__ __device__ inline int clamp_pos(long long v, int n) { return v < 0 ? 0 : (v >= n ? n - 1 : (int)v); }
+
+// Position of output sample o on its axis (floor and remainder).
+__host__ __device__ inline double sample_pos(const Axis& A, int o)
+{
+    return (o + 0.5) * ((double)A.n / A.m) - 0.5;
+}
+
+// Input samples of the group whose first output sample is o: [first, last].
+__host__ __device__ inline void group_span(const Axis& A, int o, int& first, int& last)
+{
+    const int e = o + kGroup - 1 < A.m ? o + kGroup - 1 : A.m - 1;
+    first = clamp_pos((long long)floor(sample_pos(A, o)) - 1 - kReach - A.r, A.n);
+    last = clamp_pos((long long)floor(sample_pos(A, e)) + 2 + kReach + A.r, A.n);
+}
+
+constexpr int kWeightThreads = 320;
+
+// The composed weights, one block a group; blocks 0.. of axis 0, then 1, then 2.
+// limits: [0] min, [1] max (as ordered ints), [2] non-finite input seen; reset here.
+__global__ void __launch_bounds__(kWeightThreads) axis_weights_kernel(Axes X, int* limits)
+{
+    __shared__ double gauss[2 * kMaxRadius + 1], cum[2 * kMaxRadius + 1];
+    __shared__ double q[kGroup][kTaps], zp[kTaps];
+    __shared__ double total;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        limits[0] = 0x7F800000;       // +infinity, ordered
+        limits[1] = (int)0x807FFFFF;  // -infinity, ordered
+        limits[2] = 0;
+    }
+    int g = blockIdx.x, d = 0;
+    while (g >= X.a[d].groups) g -= X.a[d++].groups;
+    const Axis A = X.a[d];
+    const int r = A.r, nk = 2 * r + 1;
+    for (int k = threadIdx.x; k < nk; k += blockDim.x)
+        gauss[k] = r > 0 ? exp(-0.5 / (A.sigma * A.sigma) * (double)(k - r) * (double)(k - r)) : 1.0;
+    // spline response: the weight of a sample at a distance from its coefficient
+    const double z = -0.26794919243112270;
+    if (threadIdx.x < kTaps) {
+        double v = -6.0 * z / (1.0 - z * z), b = z;
+        for (int e = threadIdx.x; e; e >>= 1, b *= b)
+            if (e & 1) v *= b;
+        zp[threadIdx.x] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == kWeightThreads - 1) {
+        double s = 0.0;
+        for (int k = 0; k < nk; ++k) cum[k] = s += gauss[k];
+        total = s;
+    }
+    // times the cubic weight of the coefficient in the output sample
+    for (int i = threadIdx.x; i < kGroup * kTaps; i += blockDim.x) {
+        const int o = g * kGroup + i / kTaps, m = i % kTaps;
+        double v = 0.0;
+        if (o < A.m) {
+            const double x = sample_pos(A, o), t = x - floor(x), u = 1.0 - t;
+            const double w[4] = {u * u * u / 6.0, (3.0 * t * t * t - 6.0 * t * t + 4.0) / 6.0,
+                                 (-3.0 * t * t * t + 3.0 * t * t + 3.0 * t + 1.0) / 6.0, t * t * t / 6.0};
+            for (int p = 0; p < 4; ++p) v += w[p] * zp[abs(m - kReach - p)];
+        }
+        q[i / kTaps][m] = v;
+    }
+    __syncthreads();
+    const double norm = 1.0 / total;
+    int first, last;
+    group_span(A, g * kGroup, first, last);
+    if (threadIdx.x == 0) A.start[g] = first;
+    float* out = reinterpret_cast<float*>(A.weight + (long long)g * A.span);
+    for (int i = threadIdx.x; i < A.span * kGroup; i += blockDim.x) {
+        const int c = first + i / kGroup, j = i % kGroup, o = g * kGroup + j;
+        double v = 0.0;
+        if (o < A.m && c <= last) {
+            const long long f0 = (long long)floor(sample_pos(A, o)) - 1 - kReach;
+            int m0 = 0, m1 = kTaps;  // away from the ends only samples within r of c
+            if (f0 >= 0 && f0 + kTaps <= A.n && c > 0 && c < A.n - 1) {
+                m0 = max(0, (int)(c - r - f0));
+                m1 = min(kTaps, (int)(c + r - f0) + 1);
+            }
+            for (int m = m0; m < m1; ++m) {
+                // weight of input sample c in the Gaussian at sample f, whose
+                // taps past an end all fall on that end
+                const int f = clamp_pos(f0 + m, A.n), k = c - f + r;
+                double gw = 0.0;
+                if (A.n == 1) gw = total;
+                else if (c == 0) gw = k < 0 ? 0.0 : (k >= nk ? total : cum[k]);
+                else if (c == A.n - 1) gw = k >= nk ? 0.0 : (k <= 0 ? total : total - cum[k - 1]);
+                else if (k >= 0 && k < nk) gw = gauss[k];
+                v += q[j][m] * gw;
+            }
+            v *= norm;
+        }
+        out[i] = (float)v;
+    }
+}
+
+// Order-preserving int of a float (NaN not compared).
+__device__ __forceinline__ int ordered(float v)
+{
+    const int b = __float_as_int(v);
+    return b < 0 ? b ^ 0x7FFFFFFF : b;
+}
+__device__ __forceinline__ float from_ordered(int b) { return __int_as_float(b < 0 ? b ^ 0x7FFFFFFF : b); }
+
+struct Crop {
+    const float* image;
+    Dims image_dims, dims;
+    int start[3], before[3];
+    // window sample i of axis d in the image, or -1
+    __device__ __forceinline__ int at(int d, int i) const
+    {
+        const int p = i - before[d] + start[d];
+        return p >= 0 && p < image_dims.n[d] ? p : -1;
+    }
+};
+
+__device__ __forceinline__ void copy_async4(float* dst, const float* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+constexpr int kLineThreads = 128;
+
+// The last (contiguous) axis, read from the image through the crop window: a
+// block takes kLines lines, stages the samples of as many groups as fit and
+// computes them lane = line, four outputs a sample read.  Also the window's
+// minimum, maximum and whether it is finite.  Bound by the latency of its
+// shared-memory and weight loads (11 weights a sample; issue 40%, L1 69%), at
+// 0.8 TB/s of the window: 0.18 ms for 376x376x240 samples.
+__global__ void __launch_bounds__(kLineThreads) line_axis_kernel(Crop K, Axis A, float* __restrict__ out, int* limits)
+{
+    extern __shared__ float xs[];  // [position][kLines + 1]
+    constexpr int kWarps = kLineThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long lines = (long long)K.dims.n[0] * K.dims.n[1], line0 = (long long)blockIdx.x * kLines;
+    float lo = INFINITY, hi = -INFINITY;
+    bool finite = true;
+    for (int g0 = 0; g0 < A.groups;) {
+        const int p0 = A.start[g0];
+        int g1 = g0 + 1;
+        while (g1 < A.groups && A.start[g1] + A.span - p0 <= kLinePos) ++g1;
+        const int p1 = min(A.n, A.start[g1 - 1] + A.span);
+        __syncthreads();
+        for (int l = warp; l < kLines; l += kWarps) {
+            const long long line = line0 + l;
+            const float* src = nullptr;
+            if (line < lines) {
+                const int a = K.at(0, (int)(line / K.dims.n[1])), b = K.at(1, (int)(line % K.dims.n[1]));
+                if (a >= 0 && b >= 0)
+                    src = K.image + ((long long)a * K.image_dims.n[1] + b) * K.image_dims.n[2];
+            }
+            // asynchronous copies: all of a thread's samples are in flight at once
+            for (int p = p0 + lane; p < p1; p += 32) {
+                const int c = K.at(2, p);
+                float* dst = xs + (p - p0) * (kLines + 1) + l;
+                if (src && c >= 0) copy_async4(dst, src + c);
+                else *dst = 0.f;
+            }
+        }
+        copy_async_wait();
+        __syncthreads();
+        if (line0 + lane < lines)
+            for (int p = warp; p < p1 - p0; p += kWarps) {
+                const float v = xs[p * (kLines + 1) + lane];
+                lo = fminf(lo, v);
+                hi = fmaxf(hi, v);
+                finite &= isfinite(v);
+            }
+        for (int g = g0 + warp; g < g1; g += kWarps) {
+            const float4* w = A.weight + (long long)g * A.span;
+            const float* x = xs + (A.start[g] - p0) * (kLines + 1) + lane;
+            const int span = min(A.span, p1 - A.start[g]);
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+            for (int u = 0; u < span; ++u) {
+                const float4 c = __ldg(w + u);
+                const float v = x[u * (kLines + 1)];
+                acc.x = fmaf(c.x, v, acc.x);
+                acc.y = fmaf(c.y, v, acc.y);
+                acc.z = fmaf(c.z, v, acc.z);
+                acc.w = fmaf(c.w, v, acc.w);
+            }
+            const long long line = line0 + lane;
+            if (line < lines) {
+                float* o = out + line * A.m + g * kGroup;
+                o[0] = acc.x;
+                if (g * kGroup + 1 < A.m) o[1] = acc.y;
+                if (g * kGroup + 2 < A.m) o[2] = acc.z;
+                if (g * kGroup + 3 < A.m) o[3] = acc.w;
+            }
+        }
+        g0 = g1;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    const bool bad = __any_sync(0xffffffffu, !finite);
+    if (lane == 0) {
+        if (lo <= hi) {
+            atomicMin(limits, ordered(lo));
+            atomicMax(limits + 1, ordered(hi));
+        }
+        if (bad) atomicOr(limits + 2, 1);
+    }
+}
+
+// Minimum, maximum and finiteness of a window whose lines line_axis_kernel does
+// not read completely (a factor above the filter's length).
+__global__ void __launch_bounds__(256) crop_limits_kernel(Crop K, int* limits)
+{
+    const long long total = K.dims.count();
+    float lo = INFINITY, hi = -INFINITY;
+    bool finite = true;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+         i += (long long)gridDim.x * blockDim.x) {
+        const int c = K.at(2, (int)(i % K.dims.n[2])), b = K.at(1, (int)(i / K.dims.n[2] % K.dims.n[1])),
+                  a = K.at(0, (int)(i / ((long long)K.dims.n[2] * K.dims.n[1])));
+        const float v = a >= 0 && b >= 0 && c >= 0
+                            ? __ldg(K.image + ((long long)a * K.image_dims.n[1] + b) * K.image_dims.n[2] + c)
+                            : 0.f;
+        lo = fminf(lo, v);
+        hi = fmaxf(hi, v);
+        finite &= isfinite(v);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    const bool bad = __any_sync(0xffffffffu, !finite);
+    if ((threadIdx.x & 31) == 0) {
+        if (lo <= hi) {
+            atomicMin(limits, ordered(lo));
+            atomicMax(limits + 1, ordered(hi));
+        }
+        if (bad) atomicOr(limits + 2, 1);
+    }
+}
+
+// A strided axis: in [outer][n][inner] -> out [outer][m][inner], one thread per
+// (outer, inner) and group of outputs (blockIdx.y).  FINAL: the result, clipped
+// to [min, max] when clip is set, values below zero_below 0; a window with a
+// non-finite sample has none that is finite (every line of coefficients through
+// it would be NaN), which the clip turns into the minimum.
+template <bool FINAL>
+__global__ void __launch_bounds__(128) strided_axis_kernel(const float* __restrict__ in, float* __restrict__ out,
+                                                           long long outer, long long inner, Axis A,
+                                                           const int* __restrict__ limits, int clip, float zero_below)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= outer * inner) return;
+    const long long oi = i / inner, ii = i % inner;
+    const int g = blockIdx.y, first = A.start[g], span = min(A.span, A.n - first);
+    const float4* w = A.weight + (long long)g * A.span;
+    const float* x = in + (oi * A.n + first) * inner + ii;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int u = 0; u < span; ++u) {
+        const float4 c = __ldg(w + u);
+        const float v = __ldg(x + (long long)u * inner);
+        acc.x = fmaf(c.x, v, acc.x);
+        acc.y = fmaf(c.y, v, acc.y);
+        acc.z = fmaf(c.z, v, acc.z);
+        acc.w = fmaf(c.w, v, acc.w);
+    }
+    float r[kGroup] = {acc.x, acc.y, acc.z, acc.w};
+    if (FINAL) {
+        const float lo = clip ? from_ordered(limits[0]) : -INFINITY, hi = clip ? from_ordered(limits[1]) : INFINITY;
+        const bool bad = limits[2];
+#pragma unroll
+        for (int k = 0; k < kGroup; ++k) {
+            const float v = fminf(fmaxf(bad ? NAN : r[k], lo), hi);
+            r[k] = v < zero_below ? 0.f : v;
+        }
+    }
+    float* o = out + (oi * A.m + g * kGroup) * inner + ii;
+#pragma unroll
+    for (int k = 0; k < kGroup; ++k)
+        if (g * kGroup + k < A.m) o[k * inner] = r[k];
+}
+
 int grid_for(long long n, int threads = 256)
 {
     long long b = (n + threads - 1) / threads;
@@ -287,6 +608,79 @@ PrepLayout prep_layout(const int crop[3])
     L.weights = L.part + align256(2 * kMinmaxBlocks * sizeof(float));
     L.total = L.weights + align256(3 * (2 * kMaxRadius + 1) * sizeof(float));
     return L;
+}
+
+// Workspace of the composed form: the volumes after the last and the middle
+// axis, limits, starts and weights.
+struct ComposedLayout {
+    size_t after2, after1, limits, start[3], weight[3], total;
+};
+
+// Whether the composed form applies: its volumes fit the workspace (sized for
+// the step-by-step form; strong enlargements do not) and a group of the last
+// axis fits the staged samples (factors up to about 60).
+
+bool composed_fits(const int crop[3], const int outd[3], const int radius[3], const double sigma[3], size_t have, Axes& X,
+                   ComposedLayout& L)
+{
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = off;
+        off = align256(off + bytes);
+        return at;
+    };
+    for (int d = 0; d < 3; ++d) {
+        Axis& A = X.a[d];
+        A.n = crop[d];
+        A.m = outd[d];
+        A.r = radius[d] > 0 ? radius[d] : 0;
+        A.sigma = sigma[d];
+        A.groups = (A.m + kGroup - 1) / kGroup;
+        const double want = kTaps + 2.0 * A.r + 3.0 * (double)A.n / A.m + 2.0;  // samples a group can take
+        A.span = want < A.n ? (int)want : A.n;
+        if (A.groups > 65535) return false;
+    }
+    // a group of the last axis has to fit the staged samples
+    if (X.a[2].span > kLinePos) return false;
+    L.after2 = take(sizeof(float) * (size_t)crop[0] * crop[1] * outd[2]);
+    L.after1 = take(sizeof(float) * (size_t)crop[0] * outd[1] * outd[2]);
+    L.limits = take(3 * sizeof(int));
+    for (int d = 0; d < 3; ++d) {
+        L.start[d] = take(sizeof(int) * X.a[d].groups);
+        L.weight[d] = take(sizeof(float4) * (size_t)X.a[d].groups * X.a[d].span);
+    }
+    L.total = off;
+    return off <= have;
+}
+
+int composed_downscale(const Crop& K, Axes& X, const ComposedLayout& L, int clip, float zero_below, float* out,
+                       unsigned char* ws, cudaStream_t st)
+{
+    for (int d = 0; d < 3; ++d) {
+        X.a[d].start = (int*)(ws + L.start[d]);
+        X.a[d].weight = (float4*)(ws + L.weight[d]);
+    }
+    int* limits = (int*)(ws + L.limits);
+    float *after2 = (float*)(ws + L.after2), *after1 = (float*)(ws + L.after1);
+    axis_weights_kernel<<<X.a[0].groups + X.a[1].groups + X.a[2].groups, kWeightThreads, 0, st>>>(X, limits);
+    const size_t smem = sizeof(float) * kLinePos * (kLines + 1);
+    if (cudaFuncSetAttribute((const void*)line_axis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+        return sss_set_error(SSS_ERR_CUDA, "sss_crop_downscale: %zu bytes of shared memory refused", smem);
+    const long long lines = (long long)K.dims.n[0] * K.dims.n[1];
+    const int used = X.a[2].n < kLinePos ? X.a[2].n : kLinePos;
+    line_axis_kernel<<<(unsigned)((lines + kLines - 1) / kLines), kLineThreads, sizeof(float) * used * (kLines + 1), st>>>(
+        K, X.a[2], after2, limits);
+    // lines with gaps between the groups' samples: the limits need a pass of their own
+    if ((double)X.a[2].n / X.a[2].m > kTaps)
+        crop_limits_kernel<<<grid_for(K.dims.count()), 256, 0, st>>>(K, limits);
+    auto strided = [&](auto kern, const float* in, float* to, long long outer, long long inner, const Axis& A) {
+        kern<<<dim3((unsigned)((outer * inner + 127) / 128), (unsigned)A.groups), 128, 0, st>>>(in, to, outer, inner, A,
+                                                                                              limits, clip, zero_below);
+    };
+    strided(strided_axis_kernel<false>, after2, after1, X.a[0].n, X.a[2].m, X.a[1]);
+    strided(strided_axis_kernel<true>, after1, out, 1, (long long)X.a[1].m * X.a[2].m, X.a[0]);
+    return sss_check_launch("sss_crop_downscale");
 }
 
 }  // namespace
@@ -329,18 +723,36 @@ extern "C" int sss_crop_downscale(const float* image, const int image_dims[3], c
     const Dims dp = {{crop_dims[0] + 2 * kPad, crop_dims[1] + 2 * kPad, crop_dims[2] + 2 * kPad}};
     const Dims dout = {{out_dims[0], out_dims[1], out_dims[2]}};
 
-    // Gaussian weights (FP64, normalised, then rounded to FP32) for every axis filtered
-    float hw[3][2 * kMaxRadius + 1];
     int radius[3];
     for (int d = 0; d < 3; ++d) {
         radius[d] = -1;
         if (sigma[d] <= 1e-15) continue;  // axes with a zero sigma are left unfiltered
-        const int r = (int)(4.0 * sigma[d] + 0.5);
-        if (r > kMaxRadius) return sss_set_error(SSS_ERR_INVALID, "sss_crop_downscale: kernel radius %d", r);
+        radius[d] = (int)(4.0 * sigma[d] + 0.5);
+        if (radius[d] > kMaxRadius)
+            return sss_set_error(SSS_ERR_INVALID, "sss_crop_downscale: kernel radius %d", radius[d]);
+    }
+    Axes X;
+    ComposedLayout CL;
+    if ((uintptr_t)workspace % 16 == 0 && composed_fits(crop_dims, out_dims, radius, sigma, workspace_bytes, X, CL)) {
+        Crop K;
+        K.image = image;
+        K.image_dims = din;
+        K.dims = dc;
+        for (int d = 0; d < 3; ++d) {
+            K.start[d] = crop_start[d];
+            K.before[d] = crop_before[d];
+        }
+        return composed_downscale(K, X, CL, clip, zero_below, out, ws, st);
+    }
+
+    // Gaussian weights (FP64, normalised, then rounded to FP32) for every axis filtered
+    float hw[3][2 * kMaxRadius + 1];
+    for (int d = 0; d < 3; ++d) {
+        if (radius[d] < 0) continue;
+        const int r = radius[d];
         double sum = 0.0, tmpw[2 * kMaxRadius + 1];
         for (int k = -r; k <= r; ++k) sum += (tmpw[k + r] = exp(-0.5 / (sigma[d] * sigma[d]) * k * k));
         for (int k = 0; k <= 2 * r; ++k) hw[d][k] = (float)(tmpw[k] / sum);
-        radius[d] = r;
     }
     for (int d = 0; d < 3; ++d)
         if (radius[d] >= 0 &&
