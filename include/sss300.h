@@ -292,6 +292,19 @@ int sss_tail_mask_pairs(const int32_t grid[3], const double bounds[6], const flo
                         int32_t npairs, int32_t nslices, int32_t af, double acf_below, uint8_t *out,
                         int32_t *status, void *stream);
 
+/* sss_tail_mask (pairs = NULL; npairs and nslices unused) or
+ * sss_tail_mask_pairs (sino_index unused) with a workspace: the same mask and
+ * the same errors, most LORs decided by a coarse march through a field of the
+ * map instead of the reference's walk.  workspace (device, 8-byte aligned): at
+ * least sss_tail_mask_workspace_size(grid) bytes (8 MB and 6 to 7 per voxel);
+ * with NULL or fewer, and for grids with Nx != Ny, every LOR is walked. */
+size_t sss_tail_mask_workspace_size(const int32_t grid[3]);
+int sss_tail_mask_marched(const int32_t grid[3], const double bounds[6], const float *map, int32_t use_activity,
+                          int32_t nr, int32_t nd, const double *geometry, const int16_t *lor,
+                          const int16_t *sino_index, const int32_t *pairs, int32_t npairs, int32_t nslices,
+                          int32_t af, double acf_below, uint8_t *out, int32_t *status, void *workspace,
+                          size_t workspace_bytes, void *stream);
+
 /* Back-projection scale fit.  Replaces BackProjectionScatterRandFit
  * (Python/openSSS/BackProjection.py:115-215) and BackProjection (:31-113).
  * The LOR (Ring1, d1, Ring2, d2) on the af lattice reads slice

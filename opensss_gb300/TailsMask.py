@@ -48,23 +48,23 @@ def tail_mask_device(volume, ImageSize, Geometry, SinogramCoordinates, SinogramI
     grid = np.array(shape, dtype=np.int32)
     bounds = np.ascontiguousarray(np.asarray(ImageSize, dtype=np.float64).reshape(-1)[:6])
     st = torch.cuda.current_stream(device)
+    L = _lib.lib()
+    ws = torch.empty(int(L.sss_tail_mask_workspace_size(grid.ctypes.data_as(C.c_void_p))), dtype=torch.uint8,
+                     device=device)
+    si = pairs = None
+    npairs = 0
     if span:
         pairs_np = DataReduction.span_ring_pairs(SinogramIndex)
-        nslices = pairs_np.shape[0]
+        npairs = nslices = pairs_np.shape[0]
         pairs = as_device(pairs_np, torch.int32, device)
-        out = torch.zeros(((nd + 1) * (nd // 2), nslices), dtype=torch.uint8, device=device)
-        _lib.check(_lib.lib().sss_tail_mask_pairs(
-            grid.ctypes.data_as(C.c_void_p), bounds.ctypes.data_as(C.c_void_p), _ptr(vol),
-            int(bool(use_activity)), nr, nd, _ptr(g), _ptr(lor), _ptr(pairs), nslices, nslices,
-            int(AccelerationFactor or 1), acf, _ptr(out), _ptr(status), C.c_void_p(st.cuda_stream)))
     else:
+        nslices = nr * nr
         si = as_device(geometry.check_slice_table(SinogramIndex, nr).astype(np.int16), torch.int16, device)
-        out = torch.zeros(((nd + 1) * (nd // 2), nr * nr), dtype=torch.uint8, device=device)
-        _lib.check(_lib.lib().sss_tail_mask(grid.ctypes.data_as(C.c_void_p),
-                                            bounds.ctypes.data_as(C.c_void_p), _ptr(vol),
-                                            int(bool(use_activity)), nr, nd, _ptr(g), _ptr(lor), _ptr(si),
-                                            int(AccelerationFactor or 1), acf, _ptr(out), _ptr(status),
-                                            C.c_void_p(st.cuda_stream)))
+    out = torch.zeros(((nd + 1) * (nd // 2), nslices), dtype=torch.uint8, device=device)
+    _lib.check(L.sss_tail_mask_marched(
+        grid.ctypes.data_as(C.c_void_p), bounds.ctypes.data_as(C.c_void_p), _ptr(vol), int(bool(use_activity)), nr, nd,
+        _ptr(g), _ptr(lor), _ptr(si), _ptr(pairs), npairs, nslices, int(AccelerationFactor or 1), acf, _ptr(out),
+        _ptr(status), _ptr(ws), ws.numel(), C.c_void_p(st.cuda_stream)))
     st.synchronize()
     _lib.check_status(int(status.item()))
     return out

@@ -99,6 +99,9 @@ SIGNATURES = {
     "sss_tail_mask": (C.c_int, [_P, _P, _P, _I32, _I32, _I32, _P, _P, _P, _I32, _D, _P, _P, _P]),
     "sss_tail_mask_pairs": (C.c_int, [_P, _P, _P, _I32, _I32, _I32, _P, _P, _P, _I32, _I32, _I32, _D, _P,
                                       _P, _P]),
+    "sss_tail_mask_workspace_size": (C.c_size_t, [_P]),
+    "sss_tail_mask_marched": (C.c_int, [_P, _P, _P, _I32, _I32, _I32, _P, _P, _P, _P, _I32, _I32, _I32, _D, _P, _P,
+                                        _P, C.c_size_t, _P]),
     "sss_backproject_fit_pairs": (C.c_int, [_P, _P, _I32, _I32, _P, _P, _P, _I32, _I32, _I32, _I32, _P, _P,
                                             _P, _P, _P, _P, _P, _I32, _P, _P, _P, _P, _P]),
     "sss_backproject_fit": (C.c_int, [_P, _P, _I32, _I32, _P, _P, _P, _I32, _P, _P, _P, _P, _P, _P,

@@ -6,14 +6,17 @@
 //    sampled value at cell_src[cell] + ring_off[ring_idx[slice]] (clamped at
 //    0 like fill_with_interp1d, :163), optionally summed over TOF bins in bin
 //    order (:317).  HBM-write bound.
-//  * mask_kernel: MaskDetectors (Python/openSSS/TailsMask.py:84-163): one
-//    thread per LOR on the AccelerationFactor lattice, FP64 walk and FP64
-//    line integral, mask = (1/exp(-sum) == 1).
+//  * mask_march_kernel, mask_kernel: MaskDetectors (Python/openSSS/TailsMask.py:
+//    84-163) for the LORs on the AccelerationFactor lattice: FP64 walk and FP64
+//    line integral, mask = (1/exp(-sum) == 1); the march decides most LORs
+//    without the walk.
 //  * bp_kernel + fit_reduce_kernel + fit_final_kernel: BackProjection and
 //    BackProjectionScatterRandFit (Python/openSSS/BackProjection.py:31-215):
 //    one thread per LOR, FP32 atomic scatter-add of P/n, S/n, R/n and 1 into
 //    four images, then per voxel Sbp = S/sens, T = max(P/sens - R/sens, 0)
 //    and the slope sum(x T)/sum(x^2) in FP64 with x = float(Sbp * 1e10).
+#include <limits.h>
+
 #include "common.cuh"
 #include "trace.cuh"
 
@@ -164,20 +167,11 @@ __global__ void map_sign_kernel(const float* __restrict__ map, long long n, int3
     if (__syncthreads_or(signed_value) && threadIdx.x == 0) atomicOr(status, kNoteMapSigned);
 }
 
-__global__ void __launch_bounds__(128) mask_kernel(MaskParams P)
+// The tail rule of one LOR, by the reference's walk (TailsMask.py:129-161).
+__device__ __forceinline__ bool exact_tail(const MaskParams& P, int r1, int d1, int r2, int d2, bool nonneg)
 {
-    const long long n = (long long)(P.pairs ? P.npairs : P.nr * P.nr) * P.na * P.na;
-    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    const LorRef L = lor_ref(id, P.nr, P.na, P.sino, P.pairs, P.npairs);
-    const int d1 = L.i1 * P.af, d2 = L.i2 * P.af;
-    if ((d1 == d2 && L.r1 == L.r2) || d1 > d2) return;  // TailsMask.py:129, :273
-    if (!lor_ref_ok(L, P.nr, P.nslices)) {  // the caller's slice or ring-pair table
-        raise_error(P.status, kErrTable);
-        return;
-    }
     double lc[6];
-    lor_line(P.geom, P.nd, L.r1, d1, L.r2, d2, lc);
+    lor_line(P.geom, P.nd, r1, d1, r2, d2, lc);
     double acf = 1.0;  // a miss gives Attenuation = 1 (:146-148)
     Ray r;
     if (ray_setup(P.g, lc, 1e-20, r)) {
@@ -188,7 +182,6 @@ __global__ void __launch_bounds__(128) mask_kernel(MaskParams P)
         // bound, or activity > 0) and the remaining lengths need not be
         // evaluated.  The walk itself always runs to the end, so an overrun is
         // still reported.
-        const bool nonneg = !(*(volatile const int32_t*)P.status & kNoteMapSigned);
         int c = ray_walk(P.g, r, P.cap, [&](int, int64_t lin, double t0, double t1) {
             const long long v = lin - 1;
             if (v < 0 || v >= P.nvox) {
@@ -211,9 +204,26 @@ __global__ void __launch_bounds__(128) mask_kernel(MaskParams P)
         else
             acf = div64(1.0, exp(-sum));  // :144-148
     }
-    // :150-161 (ACF == 1), or the caller's bound on the factor; one LOR per (cell, slice)
-    const bool tail = (P.acf_below > 0.0 && !P.use_activity) ? acf < P.acf_below : acf == 1.0;
-    if (tail) {
+    // :150-161 (ACF == 1), or the caller's bound on the factor
+    return (P.acf_below > 0.0 && !P.use_activity) ? acf < P.acf_below : acf == 1.0;
+}
+
+__device__ __forceinline__ bool map_nonneg(const MaskParams& P)
+{
+    return !(*(volatile const int32_t*)P.status & kNoteMapSigned);
+}
+
+// LOR id of the enumeration, by the reference's walk.
+__device__ __forceinline__ void walk_lor(const MaskParams& P, long long id, bool nonneg)
+{
+    const LorRef L = lor_ref(id, P.nr, P.na, P.sino, P.pairs, P.npairs);
+    const int d1 = L.i1 * P.af, d2 = L.i2 * P.af;
+    if ((d1 == d2 && L.r1 == L.r2) || d1 > d2) return;  // TailsMask.py:129, :273
+    if (!lor_ref_ok(L, P.nr, P.nslices)) {  // the caller's slice or ring-pair table
+        raise_error(P.status, kErrTable);
+        return;
+    }
+    if (exact_tail(P, L.r1, d1, L.r2, d2, nonneg)) {
         const int ang = P.lor[2 * ((long long)d1 * P.nd + d2)];
         const int rad = P.lor[2 * ((long long)d1 * P.nd + d2) + 1];
         if (rad < 0 || rad > P.nd || ang < 0 || ang >= P.nd / 2) {  // the caller's LOR table
@@ -221,7 +231,411 @@ __global__ void __launch_bounds__(128) mask_kernel(MaskParams P)
             return;
         }
         const long long cell = (long long)rad * (P.nd / 2) + ang;
-        P.out[cell * P.nslices + L.slice] = 1;
+        P.out[cell * P.nslices + L.slice] = 1;  // one LOR per (cell, slice)
+    }
+}
+
+// Every LOR by the reference's walk, one thread each.
+__global__ void __launch_bounds__(128) mask_kernel(MaskParams P)
+{
+    const long long n = (long long)(P.pairs ? P.npairs : P.nr * P.nr) * P.na * P.na;
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id < n) walk_lor(P, id, map_nonneg(P));
+}
+
+// ---- Most LORs are decided without the reference's walk.  A tail LOR meets no
+// non-zero voxel, the others run well inside the body, and both show from a
+// coarse march in FP32 through a field of the map's surroundings:
+//   field <= -1: every voxel within -field voxels (in each axis) is 0: the march
+//              may move that far;
+//   field > 0: the voxel and its 26 neighbours are all positive, the smallest
+//              being field: one voxel's move adds at least field times its length;
+//   -1 < field < 0: the voxel's own value is mu = -field / (1 + field);
+//   field = 0: a zero voxel beside a non-zero one.
+// The march is confined to where the line's xy projection has non-zero columns
+// about it and its z lies in the map's non-zero range; in the field it leaps, and
+// from the last two kinds it goes on voxel by voxel.  A LOR that meets no
+// non-zero voxel is a tail; one whose lower bound passes the rule's `decided` is
+// not.  What is left (voxels crossed near an edge, where FP32 positions do not
+// say which way; exits near one, where the walk could overrun; near-axis-parallel
+// crystal pairs) takes exact_tail.
+
+constexpr int kFieldReach = 15;
+// Undecided LORs kept for mask_rest_kernel; beyond them a block walks its own.
+constexpr int kMarchLeft = 1 << 20;
+
+struct MarchState {  // at the start of the workspace
+    int z_lo, z_hi;  // the map's non-zero range (empty: z_lo > z_hi)
+    unsigned left;   // undecided LORs counted (may pass kMarchLeft)
+    int pad;
+    unsigned long long lors[kMarchLeft];  // (i1 na + i2) << 32 | pair
+};
+// FP32 positions p + t q in voxels are within about 5 roundings of their size
+// of the walk's; positions this far (times |p| + |q|) from a voxel face are clear of it
+constexpr float kMarchEdge = 1e-6f;
+
+// Distance (Chebyshev, capped) to the nearest non-zero voxel, one axis at a time:
+// dist(v) = min over the axis of max(|offset|, previous axes' distance).
+__global__ void __launch_bounds__(256) field_distance_kernel(const float* __restrict__ map, const uint8_t* __restrict__ in,
+                                                             uint8_t* __restrict__ out, int n0, int n1, int n2, int axis)
+{
+    const int nvox = n0 * n1 * n2;
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nvox) return;
+    const int stride = axis == 0 ? 1 : (axis == 1 ? n0 : n0 * n1), n = axis == 0 ? n0 : (axis == 1 ? n1 : n2);
+    const int p = v / stride % n;
+    int best = kFieldReach + 1;
+    for (int k = max(-kFieldReach, -p); k <= min(kFieldReach, n - 1 - p); ++k) {
+        const int d = in ? in[v + k * stride] : (map[v + k * stride] != 0.f ? 0 : kFieldReach + 1);
+        best = min(best, max(abs(k), d));
+    }
+    out[v] = (uint8_t)best;
+}
+
+// columns[x + n0 y]: distance in the xy plane to the nearest column with a
+// non-zero voxel; state: the smallest and largest z of a non-zero voxel.
+__global__ void __launch_bounds__(256) column_kernel(const uint8_t* __restrict__ dist, uint8_t* __restrict__ columns,
+                                                     MarchState* state, int n0, int n1, int n2)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n0 * n1) return;
+    int best = 255, lo = INT_MAX, hi = -1;
+    for (int z = 0; z < n2; ++z) {
+        const int d = dist[c + n0 * n1 * z];
+        best = min(best, d);
+        if (d == 0) {
+            lo = min(lo, z);
+            hi = z;
+        }
+    }
+    columns[c] = (uint8_t)best;
+    if (hi >= 0) {
+        atomicMin(&state->z_lo, lo);
+        atomicMax(&state->z_hi, hi);
+    }
+}
+
+__global__ void __launch_bounds__(256) field_kernel(const float* __restrict__ map, const uint8_t* __restrict__ dist,
+                                                    float* __restrict__ field, MarchState* state, int n0, int n1, int n2)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        state->z_lo = INT_MAX;
+        state->z_hi = -1;
+        state->left = 0;
+    }
+    const int nvox = n0 * n1 * n2, v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nvox) return;
+    const int x = v % n0, y = v / n0 % n1, z = v / (n0 * n1);
+    float f = -(float)(dist[v] - 1);  // every voxel within dist - 1 is 0
+    if (dist[v] <= 1) {
+        f = 0.f;
+        if (dist[v] == 0 && x > 0 && x < n0 - 1 && y > 0 && y < n1 - 1 && z > 0 && z < n2 - 1) {
+            f = INFINITY;
+            for (int k = -1; k <= 1; ++k)
+                for (int j = -1; j <= 1; ++j)
+                    for (int i = -1; i <= 1; ++i) f = fminf(f, map[v + i + n0 * (j + n1 * k)]);
+            f = f > 0.f ? f : 0.f;
+        }
+        if (dist[v] == 0 && f == 0.f) {
+            const float mu = fminf(map[v], 1e5f);
+            f = -mu / (1.f + mu);
+        }
+    }
+    field[v] = f;
+}
+
+__device__ __forceinline__ LorRef pair_ref(const MaskParams& P, int e)
+{
+    LorRef L;
+    if (P.pairs) {
+        L.r1 = P.pairs[3 * e];
+        L.r2 = P.pairs[3 * e + 1];
+        L.slice = P.pairs[3 * e + 2];
+    } else {
+        L.r1 = e / P.nr;
+        L.r2 = e % P.nr;
+        L.slice = P.sino[e];
+    }
+    return L;
+}
+
+constexpr int kMaskThreads = 256;
+constexpr int kMaskChunk = 4096;  // ring pairs classified before the undecided ones are walked
+
+// One block a crystal pair (blockIdx.y <= blockIdx.x): its ring pairs share the
+// line's projection on the xy plane, so the box test's FP64 part and the hull are
+// found once, and the cell's row of slices is collected in shared memory and
+// written coalesced.  Bound by instruction issue (62% of the issue slots, 10.6
+// instructions a LOR): 51.6 million LORs through 64x64x48 voxels take 0.77 ms,
+// against 13.9 ms of FP64 walks.  256 threads: with 128 the per-pair prologue,
+// the same work for half as many, shows (3.6 against 2.6 ms when both still
+// walked their own undecided LORs; leaving those 43000 to mask_rest_kernel,
+// 0.1 ms, is what brought the 2.6 ms to 1.65 ms of the whole call).
+__global__ void __launch_bounds__(kMaskThreads, 3) mask_march_kernel(MaskParams P, const float* __restrict__ field,
+                                                                  const uint8_t* __restrict__ columns,
+                                                                  MarchState* state, int row_words, bool staged)
+{
+    // the cell's slices as bytes (row_words words; 0: written directly), then the rings' heights (staged)
+    extern __shared__ unsigned row[];
+    __shared__ int list[kMaskChunk];
+    __shared__ int listed, any_tail;
+    __shared__ unsigned kept;
+    __shared__ float s_line[9];  // in voxels: px, py, qx, qy; cm: lx, ly; entry and exit parameter; decided
+    __shared__ float s_hull[2];  // the parameters between which columns are not empty
+    __shared__ int s_mode;      // 0 march, 1 the projection misses the box, 2 walk every LOR
+    __shared__ int s_edge;      // the exit axis (0 x, 1 y); +2: the other axis exits near a voxel face
+    const int i1 = blockIdx.y, i2 = blockIdx.x;
+    if (i1 > i2 || !map_nonneg(P)) return;
+    const int d1 = i1 * P.af, d2 = i2 * P.af;
+    const int npairs = P.pairs ? P.npairs : P.nr * P.nr;
+    const double *g1 = P.geom + 3 * (long long)d1, *g2 = P.geom + 3 * (long long)d2;
+    const long long ring = 3 * (long long)P.nd;
+    for (int i = threadIdx.x; i < row_words; i += blockDim.x) row[i] = 0;
+    if (staged)  // the rings' heights in voxels
+        for (int r = threadIdx.x; r < P.nr; r += blockDim.x)
+            reinterpret_cast<float*>(row + row_words)[r] = (float)((P.geom[r * ring + 2] - P.g.b[2]) * P.g.ivs[2]);
+    // Rings may differ in their crystals' x and y: then nothing is shared.
+    if (threadIdx.x == 0) {
+        listed = any_tail = 0;
+        s_mode = 0;
+    }
+    __syncthreads();
+    const double x1 = g1[0], y1 = g1[1], x2 = g2[0], y2 = g2[1];
+    bool same = true;
+    for (int r = threadIdx.x; r < P.nr; r += blockDim.x)
+        same &= g1[r * ring] == x1 && g1[r * ring + 1] == y1 && g2[r * ring] == x2 && g2[r * ring + 1] == y2;
+    if (!__syncthreads_and(same) && threadIdx.x == 0) s_mode = 2;
+    __syncthreads();
+    if (threadIdx.x == 0 && s_mode == 0) {
+        // the xy part of the reference's box test, operation for operation
+        const double vx = sub64(x2, x1), vy = sub64(y2, y1);
+        const double xd = div64(1.0, add64(vx, 1e-20)), yd = div64(1.0, add64(vy, 1e-20));
+        const double xa = mul64(sub64(P.g.b[0], x1), xd), xb = mul64(sub64(P.g.b[3], x1), xd);
+        const double ya = mul64(sub64(P.g.b[1], y1), yd), yb = mul64(sub64(P.g.b[4], y1), yd);
+        const double xlo = xd >= 0 ? xa : xb, xhi = xd >= 0 ? xb : xa, ylo = yd >= 0 ? ya : yb, yhi = yd >= 0 ? yb : ya;
+        const double t0 = xlo > ylo ? xlo : ylo, t1 = xhi < yhi ? xhi : yhi;
+        if (xlo <= xhi && ylo <= yhi && (xlo > yhi || ylo > xhi || t0 >= 1.0 || t1 <= 0.0)) {
+            s_mode = 1;  // whatever its z does (a crystal with itself, too)
+        } else if (!(fabs(vx) > 1e-3 && fabs(vy) > 1e-3 && t0 > 1e-3 && t1 < 1.0 - 1e-3 && t1 - t0 > 1e-6)) {
+            s_mode = 2;  // near an axis' direction, an end near or in the box, a corner
+        } else {
+            s_line[0] = (float)((x1 - P.g.b[0]) * P.g.ivs[0]);
+            s_line[1] = (float)((y1 - P.g.b[1]) * P.g.ivs[1]);
+            s_line[2] = (float)(vx * P.g.ivs[0]);
+            s_line[3] = (float)(vy * P.g.ivs[1]);
+            s_line[4] = (float)vx;
+            s_line[5] = (float)vy;
+            s_line[6] = (float)t0;
+            s_line[7] = (float)t1;
+            s_line[8] = (float)(P.decided * 1.001);
+            // the other axis' exit position, in voxels
+            const bool xexit = xhi < yhi;
+            const double other = xexit ? (y1 + t1 * vy - P.g.b[1]) * P.g.ivs[1] : (x1 + t1 * vx - P.g.b[0]) * P.g.ivs[0];
+            s_edge = (xexit ? 0 : 1) + (fabs(other - rint(other)) < 1e-4 ? 2 : 0);
+        }
+    }
+    __syncthreads();
+    const int mode = s_mode, edge = s_edge;
+    const int ang = P.lor[2 * ((long long)d1 * P.nd + d2)], rad = P.lor[2 * ((long long)d1 * P.nd + d2) + 1];
+    const bool cell_ok = rad >= 0 && rad <= P.nd && ang >= 0 && ang < P.nd / 2;
+    const long long cell = (long long)rad * (P.nd / 2) + ang;
+    auto mark = [&](int slice) {
+        if (!cell_ok) any_tail = 1;
+        else if (row_words) reinterpret_cast<uint8_t*>(row)[slice] = 1;
+        else P.out[cell * P.nslices + slice] = 1;
+    };
+    // the line in voxel units, relative to the grid
+    const float vsz = (float)P.g.vs[2];
+    const float px = s_line[0], py = s_line[1], qx = s_line[2], qy = s_line[3], lx = s_line[4], ly = s_line[5];
+    const float t_in = s_line[6], t_out = s_line[7], decided = s_line[8], iqx = 1.0f / qx, iqy = 1.0f / qy;
+    const float eps_xy = kMarchEdge * fmaxf(fabsf(px) + fabsf(qx), fabsf(py) + fabsf(qy));
+    if (mode == 0 && (threadIdx.x == 0 || threadIdx.x == 32)) {
+        // from either end through the empty columns, leaping their distance
+        const bool back = threadIdx.x != 0;
+        const float dt1 = (back ? -1.0f : 1.0f) / fmaxf(fabsf(qx), fabsf(qy));
+        float t = back ? t_out : t_in;
+        for (int step = 0; step < 2 * P.cap; ++step) {
+            const int ix = min(max((int)fmaf(t, qx, px), 0), P.g.nx - 1), iy = min(max((int)fmaf(t, qy, py), 0), P.g.ny - 1);
+            const int d = columns[ix + P.g.nx * iy];
+            if (d <= 1 || (back ? t <= t_in : t >= t_out)) break;
+            t = fmaf((float)(d - 1) - 0.02f, dt1, t);
+        }
+        s_hull[back] = t;
+    }
+    __syncthreads();
+    const float h_in = s_hull[0], h_out = s_hull[1];
+    const float z_lo = (float)state->z_lo - 0.02f, z_hi = (float)state->z_hi + 1.02f;  // empty map: lo > hi
+    const float* const heights = reinterpret_cast<const float*>(row + row_words);
+    auto ring_z = [&](int r) {
+        return staged ? heights[r] : (float)((P.geom[r * ring + 2] - P.g.b[2]) * P.g.ivs[2]);
+    };
+    for (int e0 = 0; e0 < npairs; e0 += kMaskChunk) {
+        const int e1 = min(npairs, e0 + kMaskChunk);
+        for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+            const LorRef L = pair_ref(P, e);
+            if (d1 == d2 && L.r1 == L.r2) continue;  // TailsMask.py:129, :273
+            if ((unsigned)L.slice >= (unsigned)P.nslices || (unsigned)L.r1 >= (unsigned)P.nr ||
+                (unsigned)L.r2 >= (unsigned)P.nr) {  // the caller's slice or ring-pair table
+                raise_error(P.status, kErrTable);
+                continue;
+            }
+            int verdict = mode == 1 ? 1 : 2;  // 0 not a tail, 1 tail, 2 undecided
+            if (mode == 0) {
+                // ring heights in voxels
+                const float pz = ring_z(L.r1), qz = ring_z(L.r2) - pz, nz = (float)P.g.nz;
+                const float edge_eps = fmaxf(eps_xy, kMarchEdge * (fabsf(pz) + fabsf(qz)));
+                auto near_face = [&](float c) { return fabsf(c - rintf(c)) < edge_eps; };
+                float ta = t_in, tb = t_out, iqz = 0.f;
+                bool z_exit = false, clear = true;
+                if (qz == 0.f) {
+                    // a level line: exactly, and off the voxel faces, or undecided
+                    clear = P.geom[L.r1 * ring + 2] == P.geom[L.r2 * ring + 2] && !near_face(pz);
+                    if (clear && (pz < 0.f || pz > nz)) {
+                        verdict = 1;
+                        clear = false;
+                    }
+                } else {
+                    iqz = 1.0f / qz;
+                    const float za = -pz * iqz, zb = (nz - pz) * iqz;
+                    ta = fmaxf(ta, fminf(za, zb));
+                    const float zt = fmaxf(za, zb);
+                    if (zt < tb) {
+                        tb = zt;
+                        z_exit = true;
+                    }
+                }
+                const float speed = fmaxf(fmaxf(fabsf(qx), fabsf(qy)), fabsf(qz));  // voxels per unit t
+                if (clear && (ta - tb) * speed > edge_eps) {
+                    verdict = 1;  // passes the grid by
+                } else if (clear && (tb - ta) * speed > edge_eps) {
+                    // no walk exits near a voxel face of another axis, so none can overrun
+                    const bool risky = z_exit ? near_face(fmaf(tb, qx, px)) || near_face(fmaf(tb, qy, py))
+                                              : (edge & 2) || (qz != 0.f && near_face(fmaf(tb, qz, pz)));
+                    if (!risky) {
+                        const float lz = qz * vsz, len = sqrtf(lx * lx + ly * ly + lz * lz);
+                        const float dt1 = 1.0f / speed;
+                        // where a non-zero voxel can be met
+                        float t = fmaxf(ta, h_in), end = fminf(tb, h_out);
+                        if (qz != 0.f) {
+                            const float za = (z_lo - pz) * iqz, zb = (z_hi - pz) * iqz;
+                            t = fmaxf(t, fminf(za, zb));
+                            end = fminf(end, fmaxf(za, zb));
+                        } else if (pz < z_lo || pz > z_hi) {
+                            end = t;
+                        }
+                        if (z_lo > z_hi || t >= end) {
+                            mark(L.slice);
+                            continue;
+                        }
+                        float lower = 0.f;
+                        bool touched = false, placed = false;
+                        int ix = 0, iy = 0, iz = 0;
+                        for (int step = 0; step < 2 * P.cap; ++step) {
+                            if (!placed) {
+                                ix = min(max((int)fmaf(t, qx, px), 0), P.g.nx - 1);
+                                iy = min(max((int)fmaf(t, qy, py), 0), P.g.ny - 1);
+                                iz = min(max((int)fmaf(t, qz, pz), 0), P.g.nz - 1);
+                            }
+                            const float f = __ldg(field + ix + P.g.nx * (iy + P.g.ny * iz));
+                            placed = false;
+                            if (f <= -1.f) {
+                                t = fmaf(-f - 0.02f, dt1, t);
+                            } else if (f > 0.f) {
+                                touched = true;
+                                lower = fmaf(f, fminf(0.98f * dt1, end - t) * len, lower);
+                                t = fmaf(0.98f, dt1, t);
+                            } else {
+                                // to the voxel's exit
+                                const float tx = ((float)(ix + (qx > 0.f)) - px) * iqx, ty = ((float)(iy + (qy > 0.f)) - py) * iqy;
+                                const float tz = qz != 0.f ? ((float)(iz + (qz > 0.f)) - pz) * iqz : INFINITY;
+                                const float t1 = fminf(fminf(tx, ty), tz);
+                                const bool bx = t1 == tx, by = !bx && t1 == ty, bz = !bx && !by;
+                                // near an edge the walk may take either neighbour
+                                touched |= (!bx && near_face(fmaf(t1, qx, px))) || (!by && near_face(fmaf(t1, qy, py))) ||
+                                           (!bz && qz != 0.f && near_face(fmaf(t1, qz, pz)));
+                                if (f < 0.f) {
+                                    touched = true;
+                                    const float slack = edge_eps * fabsf(bx ? iqx : (by ? iqy : iqz));
+                                    const float in = fminf(t1, end) - t - slack;
+                                    if (in > 0.f) lower = fmaf(-f / (1.f + f), in * len, lower);
+                                }
+                                ix += bx ? (qx > 0.f ? 1 : -1) : 0;
+                                iy += by ? (qy > 0.f ? 1 : -1) : 0;
+                                iz += bz ? (qz > 0.f ? 1 : -1) : 0;
+                                t = (unsigned)ix < (unsigned)P.g.nx && (unsigned)iy < (unsigned)P.g.ny &&
+                                            (unsigned)iz < (unsigned)P.g.nz
+                                        ? fmaxf(t, t1)
+                                        : end;
+                                placed = true;
+                            }
+                            if (lower > decided) {
+                                verdict = 0;
+                                break;
+                            }
+                            if (t >= end) {
+                                verdict = touched ? 2 : 1;
+                                break;
+                            }
+                        }
+                    }
+                }
+            }
+            if (verdict == 1) mark(L.slice);
+            if (verdict == 2) list[atomicAdd(&listed, 1)] = e;
+        }
+        __syncthreads();
+        const int n = listed;
+        if (threadIdx.x == 0 && n)  // counted on a little beyond the list only
+            kept = *(volatile unsigned*)&state->left < kMarchLeft ? atomicAdd(&state->left, (unsigned)n) : kMarchLeft;
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            if (kept < kMarchLeft && i < (int)(kMarchLeft - kept)) {
+                state->lors[kept + i] = (unsigned long long)((unsigned)i1 * (unsigned)P.na + i2) << 32 | (unsigned)list[i];
+                continue;
+            }
+            const LorRef L = pair_ref(P, list[i]);
+            if (exact_tail(P, L.r1, d1, L.r2, d2, true)) mark(L.slice);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) listed = 0;
+        __syncthreads();
+    }
+    if (any_tail && threadIdx.x == 0) raise_error(P.status, kErrTable);  // the caller's LOR table
+    if (cell_ok && row_words) {
+        unsigned* out = reinterpret_cast<unsigned*>(P.out + cell * P.nslices);
+        for (int i = threadIdx.x; i < row_words; i += blockDim.x)
+            if (row[i]) atomicOr(out + i, row[i]);  // other cells' bytes stay as they are
+    }
+}
+
+constexpr int kRestChunk = 2048;
+
+// The undecided LORs, by the reference's walk; every LOR where the map has a
+// negative or NaN value (no sum only grows then, and nothing was marched).
+__global__ void __launch_bounds__(64) mask_rest_kernel(MaskParams P, MarchState* state)
+{
+    if (!map_nonneg(P)) {
+        const long long n = (long long)(P.pairs ? P.npairs : P.nr * P.nr) * P.na * P.na;
+        __shared__ unsigned chunk;
+        for (;;) {  // nothing was listed: the count hands out chunks
+            __syncthreads();
+            if (threadIdx.x == 0) chunk = atomicAdd(&state->left, 1u);
+            __syncthreads();
+            const long long first = (long long)chunk * kRestChunk;
+            if (first >= n) return;
+            for (long long id = first + threadIdx.x; id < min(n, first + kRestChunk); id += blockDim.x) walk_lor(P, id, false);
+        }
+    }
+    const unsigned n = min(state->left, (unsigned)kMarchLeft);
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned long long id = state->lors[i];
+        const unsigned cross = (unsigned)(id >> 32), na = (unsigned)P.na;
+        const int e = (int)(unsigned)id, d1 = (int)(cross / na) * P.af, d2 = (int)(cross % na) * P.af;
+        const LorRef L = pair_ref(P, e);
+        if (!exact_tail(P, L.r1, d1, L.r2, d2, true)) continue;
+        const int ang = P.lor[2 * ((long long)d1 * P.nd + d2)], rad = P.lor[2 * ((long long)d1 * P.nd + d2) + 1];
+        if (rad < 0 || rad > P.nd || ang < 0 || ang >= P.nd / 2) raise_error(P.status, kErrTable);
+        else P.out[((long long)rad * (P.nd / 2) + ang) * P.nslices + L.slice] = 1;
     }
 }
 
@@ -572,7 +986,7 @@ namespace {
 int tail_mask(const int32_t grid[3], const double bounds[6], const float* map, int32_t use_activity, int32_t nr,
               int32_t nd, const double* geometry, const int16_t* lor, const int16_t* sino_index,
               const int32_t* pairs, int32_t npairs, int32_t nslices, int32_t af, double acf_below, uint8_t* out,
-              int32_t* status, void* stream)
+              int32_t* status, void* workspace, size_t workspace_bytes, void* stream)
 {
     if (!(acf_below == 0.0 || acf_below > 1.0))
         return sss_set_error(SSS_ERR_INVALID, "sss_tail_mask: acf_below must be 0 (ACF == 1) or above 1");
@@ -605,11 +1019,62 @@ int tail_mask(const int32_t grid[3], const double bounds[6], const float* map, i
     map_sign_kernel<<<(unsigned)(nb < 1024 ? nb : 1024), 256, 0, (cudaStream_t)stream>>>(map, P.nvox, status);
     int rc = sss_check_launch("map_sign_kernel");
     if (rc) return rc;
+    // The march needs the field in the workspace and a map whose linear index is
+    // that of its voxel (nx == ny); walking every LOR takes 14.5 ms for 51.6
+    // million LORs through 64x64x48 voxels, marching first 1.65 ms (0.46 ms of
+    // either zero-fills the mask).
+    if (workspace && (uintptr_t)workspace % 8 == 0 &&
+        workspace_bytes >= sss_tail_mask_workspace_size(grid) && grid[0] == grid[1] && P.nvox < (1 << 28) &&
+        P.na <= 65535) {
+        cudaStream_t st = (cudaStream_t)stream;
+        MarchState* state = (MarchState*)workspace;
+        float* field = (float*)(state + 1);
+        uint8_t *da = (uint8_t*)(field + P.nvox), *db = da + P.nvox, *columns = db + P.nvox;
+        const unsigned fb = blocks_for(P.nvox, 256);
+        field_distance_kernel<<<fb, 256, 0, st>>>(map, nullptr, da, grid[0], grid[1], grid[2], 0);
+        field_distance_kernel<<<fb, 256, 0, st>>>(map, da, db, grid[0], grid[1], grid[2], 1);
+        field_distance_kernel<<<fb, 256, 0, st>>>(map, db, da, grid[0], grid[1], grid[2], 2);
+        field_kernel<<<fb, 256, 0, st>>>(map, da, field, state, grid[0], grid[1], grid[2]);
+        column_kernel<<<blocks_for((long long)grid[0] * grid[1], 256), 256, 0, st>>>(da, columns, state, grid[0],
+                                                                                    grid[1], grid[2]);
+        if ((rc = sss_check_launch("field_kernel"))) return rc;
+        // rows of bytes are collected in shared memory where they are whole aligned words
+        const bool rows = P.nslices % 4 == 0 && (uintptr_t)out % 4 == 0 && P.nslices <= 24 * 1024;
+        const int words = rows ? P.nslices / 4 : 0;
+        const bool staged = nr <= 1024;
+        mask_march_kernel<<<dim3((unsigned)P.na, (unsigned)P.na), kMaskThreads, 4 * (size_t)(words + (staged ? nr : 0)),
+                            st>>>(P, field, columns, state, words, staged);
+        if ((rc = sss_check_launch("mask_march_kernel"))) return rc;
+        mask_rest_kernel<<<2048, 64, 0, st>>>(P, state);
+        return sss_check_launch("mask_rest_kernel");
+    }
     mask_kernel<<<blocks_for(n, 128), 128, 0, (cudaStream_t)stream>>>(P);
     return sss_check_launch("mask_kernel");
 }
 
 }  // namespace
+
+extern "C" size_t sss_tail_mask_workspace_size(const int32_t grid[3])
+{
+    if (!grid || grid[0] < 1 || grid[1] < 1 || grid[2] < 1) return 0;
+    return sizeof(MarchState) + 6 * (size_t)grid[0] * grid[1] * grid[2] + (size_t)grid[0] * grid[1];
+}
+
+extern "C" int sss_tail_mask_marched(const int32_t grid[3], const double bounds[6], const float* map,
+                                     int32_t use_activity, int32_t nr, int32_t nd, const double* geometry,
+                                     const int16_t* lor, const int16_t* sino_index, const int32_t* pairs, int32_t npairs,
+                                     int32_t nslices, int32_t af, double acf_below, uint8_t* out, int32_t* status,
+                                     void* workspace, size_t workspace_bytes, void* stream)
+{
+    int rc = check_grid(grid, bounds, "sss_tail_mask_marched");
+    if (rc) return rc;
+    if (!map || !geometry || !lor || (!sino_index && !pairs) || !out || nr < 1 || nd < 2 || af < 1 ||
+        (pairs && (npairs < 0 || nslices < 1)) || (uintptr_t)workspace % 4 != 0)
+        return sss_set_error(SSS_ERR_INVALID, "sss_tail_mask_marched: bad argument");
+    return tail_mask(grid, bounds, map, use_activity, nr, nd, geometry, lor, pairs ? nullptr : sino_index, pairs,
+                     pairs ? npairs : 0, pairs ? nslices : 0, af, acf_below, out, status, workspace, workspace_bytes,
+                     stream);
+}
 
 extern "C" int sss_tail_mask(const int32_t grid[3], const double bounds[6], const float* map,
                              int32_t use_activity, int32_t nr, int32_t nd, const double* geometry,
@@ -621,7 +1086,7 @@ extern "C" int sss_tail_mask(const int32_t grid[3], const double bounds[6], cons
     if (!map || !geometry || !lor || !sino_index || !out || nr < 1 || nd < 2 || af < 1)
         return sss_set_error(SSS_ERR_INVALID, "sss_tail_mask: bad argument");
     return tail_mask(grid, bounds, map, use_activity, nr, nd, geometry, lor, sino_index, nullptr, 0, 0, af,
-                     acf_below, out, status, stream);
+                     acf_below, out, status, nullptr, 0, stream);
 }
 
 extern "C" int sss_tail_mask_pairs(const int32_t grid[3], const double bounds[6], const float* map,
@@ -634,7 +1099,7 @@ extern "C" int sss_tail_mask_pairs(const int32_t grid[3], const double bounds[6]
     if (!map || !geometry || !lor || !pairs || !out || nr < 1 || nd < 2 || af < 1 || npairs < 0 || nslices < 1)
         return sss_set_error(SSS_ERR_INVALID, "sss_tail_mask_pairs: bad argument");
     return tail_mask(grid, bounds, map, use_activity, nr, nd, geometry, lor, nullptr, pairs, npairs, nslices, af,
-                     acf_below, out, status, stream);
+                     acf_below, out, status, nullptr, 0, stream);
 }
 
 namespace {
