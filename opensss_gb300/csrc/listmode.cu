@@ -21,7 +21,7 @@ using namespace sss;
 
 struct Parsed {
     int d1, r1, d2, r2;  // crystal (unshifted, d1 < d2) and ring of each side
-    double tof;          // ps, sign for the (r1, r2) order
+    float tof;           // ps, sign for the (r1, r2) order
 };
 
 __device__ __forceinline__ uint32_t load_u32(const unsigned char* rec, int off)
@@ -38,24 +38,25 @@ __device__ __forceinline__ float load_f32(const unsigned char* rec, int off)
 __device__ __forceinline__ Parsed parse_event(const unsigned char* rec, const sss_listmode_layout& L, int ncr,
                                               int shift)
 {
-    const long long a = load_u32(rec, L.id_offset), b = load_u32(rec, L.id_offset + 4);
-    const double tof = (double)load_f32(rec, L.tof_offset);
-    const long long id1 = a < b ? a : b, id2 = a < b ? b : a;
-    const double tof_t = a < b ? tof : -tof;
+    const uint32_t a = load_u32(rec, L.id_offset), b = load_u32(rec, L.id_offset + 4);
+    const float tof = load_f32(rec, L.tof_offset);
+    const uint32_t id1 = a < b ? a : b, id2 = a < b ? b : a;
+    const float tof_t = a < b ? tof : -tof;
     Parsed P;
-    const int c1 = (int)(id1 % ncr), c2 = (int)(id2 % ncr);
+    const uint32_t q1 = id1 / (uint32_t)ncr, q2 = id2 / (uint32_t)ncr;
+    const int c1 = (int)(id1 - q1 * (uint32_t)ncr), c2 = (int)(id2 - q2 * (uint32_t)ncr);
     P.d1 = c1 < c2 ? c1 : c2;
     P.d2 = c1 < c2 ? c2 : c1;
     int s1 = c1 - shift, s2 = c2 - shift;
     if (s1 < 0) s1 += ncr;
     if (s2 < 0) s2 += ncr;
     if (s1 < s2) {
-        P.r1 = (int)(id1 / ncr);
-        P.r2 = (int)(id2 / ncr);
+        P.r1 = (int)q1;
+        P.r2 = (int)q2;
         P.tof = tof_t;
     } else {
-        P.r1 = (int)(id2 / ncr);
-        P.r2 = (int)(id1 / ncr);
+        P.r1 = (int)q2;
+        P.r2 = (int)q1;
         P.tof = -tof_t;
     }
     return P;
@@ -75,13 +76,27 @@ __device__ __forceinline__ long long event_cell(const Parsed& P, const sss_sino_
     return ((long long)rad * M.nang + ang) * M.nslices + sino;
 }
 
-// TOF bin as the reference computes it (Datafile.py:103-110); -1 = outside.
-__device__ __forceinline__ int tof_bin(double tof, const sss_sino_map& M)
+// TOF bin as the reference computes it in FP64 (Datafile.py:103-110); -1 = the
+// TOF is outside the range, -2 = inside it but in no bin (the upper end).  The
+// FP64 pipe runs at about 1/70 of the FP32 rate, so the two FP64 divisions are
+// left to events near a bin edge: t below differs from the exact quotient by a
+// few FP32 roundings of tof_bins at most, well within kBinEdge * tof_bins.  (A
+// NaN TOF or quotient falls to the FP64 form, too.)
+constexpr float kBinEdge = 2e-6f;
+
+__device__ __forceinline__ int tof_bin(float tof, const sss_sino_map& M)
 {
-    if (fabs(tof) > M.tof_range) return -1;
+    const float range = (float)M.tof_range, bins = (float)M.tof_bins;
+    if (range > 1e-30f && range < 1e30f) {
+        const float t32 = (tof + range) * (bins / (2.0f * range)), edge = kBinEdge * bins;
+        if (t32 < -edge || t32 > bins + edge) return -1;
+        if (fabsf(t32 - rintf(t32)) > edge) return (int)t32;
+    }
+    const double x = (double)tof;
+    if (fabs(x) > M.tof_range) return -1;
     const double w = (2.0 * M.tof_range) / M.tof_bins;
-    const double t = (tof + M.tof_range) / w;
-    if (t < 0.0 || t >= (double)M.tof_bins) return -1;
+    const double t = (x + M.tof_range) / w;
+    if (t < 0.0 || t >= (double)M.tof_bins) return -2;
     return (int)t;
 }
 
@@ -135,25 +150,30 @@ __global__ void last_values_kernel(const unsigned char* __restrict__ ev, long lo
 
 // ------------------------------------------------------------------ injection
 
-constexpr int kInjectThreads = 256;
+constexpr int kInjectThreads = 256, kInjectItems = 4, kInjectBlock = kInjectThreads * kInjectItems;
 
 __device__ __forceinline__ bool inject_keep(const unsigned char* rec, const sss_listmode_layout& L,
                                             const sss_sino_map& M, const float* scat, const float* factor,
                                             float& rate, bool& bad)
 {
     const Parsed P = parse_event(rec, L, M.nd_lor * M.mash, M.shift);
-    if (fabs(P.tof) > M.tof_range) return false;  // :207-208, before the tables
+    const int bin = tof_bin(P.tof, M);
+    if (bin == -1) return false;  // :207-208, before the tables
     const long long cell = event_cell(P, M);
     if (cell == -2) {
         bad = true;
         return false;
     }
-    if (cell < 0) return false;
-    const int bin = tof_bin(P.tof, M);
-    if (bin < 0) return false;
+    if (cell < 0 || bin < 0) return false;
     const long long ncell = (long long)M.nrad * M.nang * M.nslices;
     rate = __fmul_rn(factor[bin], scat[bin * ncell + cell]);  // :229 in float32
     return true;
+}
+
+// Event j of a thread: a block's events in rounds of kInjectThreads, in file order.
+__device__ __forceinline__ long long inject_event(int j)
+{
+    return (long long)blockIdx.x * kInjectBlock + j * kInjectThreads + threadIdx.x;
 }
 
 __global__ void __launch_bounds__(kInjectThreads) inject_count_kernel(
@@ -161,13 +181,22 @@ __global__ void __launch_bounds__(kInjectThreads) inject_count_kernel(
     const float* __restrict__ scat, const float* __restrict__ factor, unsigned int* __restrict__ block_counts,
     int32_t* status)
 {
-    const long long e = (long long)blockIdx.x * kInjectThreads + threadIdx.x;
-    float rate;
+    __shared__ int total;
+    if (threadIdx.x == 0) total = 0;
     bool bad = false;
-    const bool keep = e < n && inject_keep(ev + e * L.record_bytes, L, M, scat, factor, rate, bad);
+    int c = 0;
+#pragma unroll
+    for (int j = 0; j < kInjectItems; ++j) {
+        const long long e = inject_event(j);
+        float rate;
+        c += e < n && inject_keep(ev + e * L.record_bytes, L, M, scat, factor, rate, bad);
+    }
     if (bad) raise_error(status, kErrEvent);
-    const int c = __syncthreads_count(keep);
-    if (threadIdx.x == 0) block_counts[blockIdx.x] = (unsigned int)c;
+    c = __reduce_add_sync(0xffffffffu, c);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) atomicAdd(&total, c);
+    __syncthreads();
+    if (threadIdx.x == 0) block_counts[blockIdx.x] = (unsigned int)total;
 }
 
 // Exclusive scan of the block counts in one block (counts are < 2^32 total
@@ -197,34 +226,54 @@ __global__ void __launch_bounds__(1024) inject_scan_kernel(const unsigned int* _
     if (threadIdx.x == 1023) *total = part[1023];
 }
 
+// Bound by memory: 19 million of 20 million events read their scatter value at
+// random from 1.4 GB, 128 bytes a miss, 3.4 GB in all in 0.62 ms (5.5 TB/s).
+// Four events a thread shorten the scan of the block counts from 72 to 17 us;
+// gathering the output rows for coalesced stores was slower (0.76 ms).
 __global__ void __launch_bounds__(kInjectThreads) inject_write_kernel(
     const unsigned char* __restrict__ ev, long long n, sss_listmode_layout L, sss_sino_map M,
     const float* __restrict__ scat, const float* __restrict__ factor,
     const unsigned long long* __restrict__ offsets, unsigned char* __restrict__ out, int out_bytes)
 {
-    __shared__ unsigned int warp_sums[kInjectThreads / 32];
-    const long long e = (long long)blockIdx.x * kInjectThreads + threadIdx.x;
-    float rate = 0.f;
-    bool bad = false;
-    const unsigned char* rec = ev + e * L.record_bytes;
-    const bool keep = e < n && inject_keep(rec, L, M, scat, factor, rate, bad);
-    // rank of this event among the block's kept events
-    const unsigned int ballot = __ballot_sync(0xffffffffu, keep);
+    constexpr int kWarps = kInjectThreads / 32;
+    __shared__ int sums[kInjectItems * kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) warp_sums[warp] = __popc(ballot);
+    float rate[kInjectItems];
+    unsigned ballot[kInjectItems];
+#pragma unroll
+    for (int j = 0; j < kInjectItems; ++j) {
+        const long long e = inject_event(j);
+        bool bad = false;
+        rate[j] = 0.f;
+        const bool keep = e < n && inject_keep(ev + e * L.record_bytes, L, M, scat, factor, rate[j], bad);
+        ballot[j] = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) sums[j * kWarps + warp] = __popc(ballot[j]);
+    }
     __syncthreads();
-    unsigned int before = 0;
-    for (int w = 0; w < warp; ++w) before += warp_sums[w];
-    before += __popc(ballot & ((1u << lane) - 1u));
-    if (!keep) return;
-    unsigned char* dst = out + (offsets[blockIdx.x] + before) * (unsigned long long)out_bytes;
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(rec);
-    uint32_t* d = reinterpret_cast<uint32_t*>(dst);
+    if (warp == 0) {  // 32 sums, in file order
+        const int own = sums[lane];
+        int s = own;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += v;
+        }
+        sums[lane] = s;
+    }
+    __syncthreads();
     const int head = L.scatter_offset / 4, words = L.record_bytes / 4;
-    for (int i = 0; i < head; ++i) d[i] = src[i];
-    d[head] = __float_as_uint(rate);
-    for (int i = head; i < words; ++i) d[i + 1] = src[i];
+    unsigned char* const block_out = out + offsets[blockIdx.x] * (unsigned long long)out_bytes;
+#pragma unroll
+    for (int j = 0; j < kInjectItems; ++j) {
+        if (!(ballot[j] >> lane & 1u)) continue;
+        const int at = sums[j * kWarps + warp] - __popc(ballot[j]) + __popc(ballot[j] & ((1u << lane) - 1u));
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(ev + inject_event(j) * L.record_bytes);
+        uint32_t* d = reinterpret_cast<uint32_t*>(block_out + (long long)at * out_bytes);
+        for (int i = 0; i < head; ++i) d[i] = src[i];
+        d[head] = __float_as_uint(rate[j]);
+        for (int i = head; i < words; ++i) d[i + 1] = src[i];
+    }
 }
+static_assert(kInjectItems * kInjectThreads / 32 == 32, "one warp scans the sums");
 
 int check_layout(const sss_listmode_layout* L, const sss_sino_map* M, const char* who)
 {
@@ -291,7 +340,7 @@ extern "C" int sss_histogram_finish(const void* events, int64_t n_events, const 
 
 extern "C" size_t sss_inject_workspace_size(int64_t n_events)
 {
-    const long long nb = (n_events + kInjectThreads - 1) / kInjectThreads;
+    const long long nb = (n_events + kInjectBlock - 1) / kInjectBlock;
     return (size_t)(((nb * 4 + 255) / 256) * 256 + ((nb * 8 + 255) / 256) * 256 + 256);
 }
 
@@ -311,7 +360,7 @@ extern "C" int sss_inject_scatters(const void* events, int64_t n_events, const s
             return sss_set_error(SSS_ERR_CUDA, "sss_inject_scatters: memset failed");
         return SSS_OK;
     }
-    const long long nb = (n_events + kInjectThreads - 1) / kInjectThreads;
+    const long long nb = (n_events + kInjectBlock - 1) / kInjectBlock;
     if (nb > 0x7fffffffLL) return sss_set_error(SSS_ERR_INVALID, "sss_inject_scatters: too many events");
     char* ws = (char*)workspace;
     unsigned int* counts = (unsigned int*)ws;
