@@ -406,6 +406,18 @@ int sss_histogram_prompts(const void *events, int64_t n_events, const sss_listmo
 int sss_histogram_finish(const void *events, int64_t n_events, const sss_listmode_layout *layout,
                          const sss_sino_map *map, const uint32_t *counts, const unsigned long long *last,
                          double duration, uint16_t *prompts, float *randoms, float *norm, void *stream);
+/* sss_histogram_prompts and sss_histogram_finish in one, by tiles of cells in
+ * shared memory: prompts, randoms and norm (the latter two may be NULL) are
+ * written whole, cells without an event as 0, 0 and 1; nothing need be zeroed.
+ * workspace (device, 16-byte aligned): at least
+ * sss_histogram_tiled_workspace_size(n_events, map, randoms || norm) bytes
+ * (24 per event, 12 without randoms and norm); that size is 0 where the tiles
+ * do not hold the problem (2^31 events, cells * (tof_bins + 1) beyond 2^32, or
+ * tens of thousands of bins), which takes the two calls above. */
+size_t sss_histogram_tiled_workspace_size(int64_t n_events, const sss_sino_map *map, int32_t want_values);
+int sss_histogram_tiled(const void *events, int64_t n_events, const sss_listmode_layout *layout,
+                        const sss_sino_map *map, double duration, uint16_t *prompts, float *randoms, float *norm,
+                        void *workspace, size_t workspace_bytes, int32_t *status, void *stream);
 /* Scatter injection: keeps the events the reference keeps, in file order,
  * each with the float32 rate factor[bin] * scatters[bin][cell] inserted at
  * scatter_offset (out_events: record_bytes + 4 per event; *out_count

@@ -74,21 +74,32 @@ def histogram_device(events: torch.Tensor, header: dict, LORCoordinates, Sinogra
     L = layout_of(header)
     M = sino_map(lor_t, lor.shape[0], mash, Shift, slices_t, nrad, nang, nslices, TOF_bins, TOF_range)
     n = events.numel() // L.record_bytes
-    counts = torch.zeros((nrad, nang, nslices, TOF_bins), dtype=torch.int32, device=device)
     want = header["random_flag"] or header["normalization_flag"]
-    last = torch.zeros((nrad, nang, nslices), dtype=torch.int64, device=device) if want else None
+    shape = (nrad, nang, nslices)
     status = torch.zeros(1, dtype=torch.int32, device=device)
     st = C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
     lib = _lib.lib()
-    _lib.check(lib.sss_histogram_prompts(_ptr(events), n, C.byref(L), C.byref(M), _ptr(counts), _ptr(last),
-                                         _ptr(status), st))
-    prompts = torch.empty((nrad, nang, nslices, TOF_bins), dtype=torch.int16, device=device)
-    randoms = (torch.zeros((nrad, nang, nslices), dtype=torch.float32, device=device)
-               if header["random_flag"] else None)
-    norm = (torch.ones((nrad, nang, nslices), dtype=torch.float32, device=device)
-            if header["normalization_flag"] else None)
-    _lib.check(lib.sss_histogram_finish(_ptr(events), n, C.byref(L), C.byref(M), _ptr(counts), _ptr(last),
-                                        float(header["duration"]), _ptr(prompts), _ptr(randoms), _ptr(norm), st))
+    prompts = torch.empty((*shape, TOF_bins), dtype=torch.int16, device=device)
+    need, ws = int(lib.sss_histogram_tiled_workspace_size(n, C.byref(M), int(bool(want)))), None
+    if need:
+        try:
+            ws = torch.empty(need, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:  # the two-pass form's memory does not grow with the events
+            pass
+    if ws is not None:
+        randoms = torch.empty(shape, dtype=torch.float32, device=device) if header["random_flag"] else None
+        norm = torch.empty(shape, dtype=torch.float32, device=device) if header["normalization_flag"] else None
+        _lib.check(lib.sss_histogram_tiled(_ptr(events), n, C.byref(L), C.byref(M), float(header["duration"]),
+                                           _ptr(prompts), _ptr(randoms), _ptr(norm), _ptr(ws), need, _ptr(status), st))
+    else:
+        counts = torch.zeros((*shape, TOF_bins), dtype=torch.int32, device=device)
+        last = torch.zeros(shape, dtype=torch.int64, device=device) if want else None
+        _lib.check(lib.sss_histogram_prompts(_ptr(events), n, C.byref(L), C.byref(M), _ptr(counts), _ptr(last),
+                                             _ptr(status), st))
+        randoms = torch.zeros(shape, dtype=torch.float32, device=device) if header["random_flag"] else None
+        norm = torch.ones(shape, dtype=torch.float32, device=device) if header["normalization_flag"] else None
+        _lib.check(lib.sss_histogram_finish(_ptr(events), n, C.byref(L), C.byref(M), _ptr(counts), _ptr(last),
+                                            float(header["duration"]), _ptr(prompts), _ptr(randoms), _ptr(norm), st))
     torch.cuda.current_stream(device).synchronize()
     _lib.check_status(int(status.item()))
     return prompts, randoms, norm

@@ -112,6 +112,9 @@ SIGNATURES = {
                                         _P, _P]),
     "sss_histogram_finish": (C.c_int, [_P, _I64, C.POINTER(ListmodeLayout), C.POINTER(SinoMap), _P, _P,
                                        _D, _P, _P, _P, _P]),
+    "sss_histogram_tiled_workspace_size": (C.c_size_t, [_I64, C.POINTER(SinoMap), _I32]),
+    "sss_histogram_tiled": (C.c_int, [_P, _I64, C.POINTER(ListmodeLayout), C.POINTER(SinoMap), _D, _P, _P, _P, _P,
+                                      C.c_size_t, _P, _P]),
     "sss_inject_workspace_size": (C.c_size_t, [_I64]),
     "sss_inject_scatters": (C.c_int, [_P, _I64, C.POINTER(ListmodeLayout), C.POINTER(SinoMap), _P, _P,
                                       _P, _P, _P, C.c_size_t, _P, _P]),
