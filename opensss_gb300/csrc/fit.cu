@@ -764,16 +764,14 @@ __global__ void __launch_bounds__(kBpThreads, NPB > 0 ? 6 : 0) bp_kernel(FitPara
     // Voxel count (the reference divides by len(Lengths), :108-110).  Every
     // step of the walk moves one voxel along one axis towards the end voxel,
     // so a walk that ends crosses 1 + |dX| + |dY| + |dZ| voxels; one that would
-    // overrun is caught by the walk below.  The length-weighted back-projection
-    // needs the summed length first (:294-297), so it walks twice.
-    double total = 0.0;
+    // overrun is caught by the walk below.
     int n_vox = 1 + abs(r.xe - r.X) + abs(r.ye - r.Y) + abs(r.ze - r.Z);
-    if (P.length_weighted) {
-        Ray r2 = r;
-        n_vox = ray_walk(P.g, r2, P.cap, [&](int, int64_t, double t0, double t1) {
-            total = add64(total, ref_length(r2, t0, t1));
-        });
-    }
+    // Length-weighted (:294-297): a voxel's share of the summed length is its
+    // share of the parameter range that the segments divide among them, so that
+    // neither the lengths nor a walk for their sum is needed.  (With both, the
+    // FP64 pipe bound the kernel, at 2.1 ms for 1.0 million LORs through 37x37x26
+    // voxels; 0.55 ms without.)
+    const double per_t = P.length_weighted ? div64(1.0, sub64(r.tmax, r.tmin)) : 0.0;
     if (n_vox < 0 || n_vox > P.cap) {
         raise_error(P.status, kErrOverrun);
         return;
@@ -846,7 +844,7 @@ __global__ void __launch_bounds__(kBpThreads, NPB > 0 ? 6 : 0) bp_kernel(FitPara
             bad = true;
             return;
         }
-        const double w = P.length_weighted ? div64(ref_length(r, t0, t1), total) : 0.0;
+        const double w = P.length_weighted ? mul64(fabs(sub64(t1, t0)), per_t) : 0.0;
         const float rw = P.length_weighted ? (float)mul64((double)rv, w) : ar;
         // (D, S) of bin b from this LOR: prompts minus randoms, and scatter
         // (one bin: the LOR's values, else re-read per voxel, L1-resident)
