@@ -46,8 +46,8 @@ def fit_device(prompts, randoms, mask, scatters, scat_cell, scat_ring, GridSize,
     nvox = int(np.prod(grid))
     images = torch.empty(8 * nvox, dtype=torch.float32, device=device)
     sums = torch.empty(2, dtype=torch.float64, device=device)
-    scale = torch.empty(1, dtype=torch.float32, device=device)
-    status = torch.zeros(1, dtype=torch.int32, device=device)
+    result = torch.zeros(2, dtype=torch.int32, device=device)  # status and scale: one read-back
+    status, scale = result[:1], result[1:].view(torch.float32)
     m_u8 = mask if mask.dtype == torch.uint8 else None
     m_f = None if m_u8 is not None else mask
     st = torch.cuda.current_stream(device)
@@ -64,9 +64,9 @@ def fit_device(prompts, randoms, mask, scatters, scat_cell, scat_ring, GridSize,
             _ptr(order), int(AccelerationFactor or 1), _ptr(prompts), _ptr(randoms), _ptr(m_f), _ptr(m_u8),
             _ptr(scatters), _ptr(cs), _ptr(rs), int(bool(scat_clamp)), _ptr(images), _ptr(sums),
             _ptr(scale), _ptr(status), C.c_void_p(st.cuda_stream)))
-    st.synchronize()
-    _lib.check_status(int(status.item()))
-    return float(scale.item())
+    host = result.cpu()
+    _lib.check_status(int(host[0]))
+    return float(host[1:].view(torch.float32))
 
 
 def fit_bins_device(prompts, randoms, mask, scatters, scat_stride: int, scat_cell, scat_ring, GridSize,
@@ -97,8 +97,8 @@ def fit_bins_device(prompts, randoms, mask, scatters, scat_stride: int, scat_cel
     nvox = int(np.prod(grid))
     images = torch.empty((nbins + 1) * 4 * nvox, dtype=torch.float32, device=device)
     sums = torch.empty(2 * nbins, dtype=torch.float64, device=device)
-    scales = torch.empty(nbins, dtype=torch.float32, device=device)
-    status = torch.zeros(1, dtype=torch.int32, device=device)
+    result = torch.zeros(1 + nbins, dtype=torch.int32, device=device)  # status and scales: one read-back
+    status, scales = result[:1], result[1:].view(torch.float32)
     m_u8 = mask if mask.dtype == torch.uint8 else None
     m_f = None if m_u8 is not None else mask
     st = torch.cuda.current_stream(device)
@@ -109,9 +109,9 @@ def fit_bins_device(prompts, randoms, mask, scatters, scat_stride: int, scat_cel
         _ptr(prompts), stride, _ptr(randoms), _ptr(m_f), _ptr(m_u8), _ptr(scatters), int(scat_stride), _ptr(cs),
         _ptr(rs), int(bool(scat_clamp)), _ptr(images), _ptr(sums), _ptr(scales), _ptr(status),
         C.c_void_p(st.cuda_stream)))
-    st.synchronize()
-    _lib.check_status(int(status.item()))
-    return scales.cpu().numpy()
+    host = result.cpu()
+    _lib.check_status(int(host[0]))
+    return host[1:].view(torch.float32).numpy()
 
 
 def BackProjectionScatterRandFit(PromptSinogram, ScatterSinogram, RandomSinogram, MaskSinogram,

@@ -100,8 +100,7 @@ def histogram_device(events: torch.Tensor, header: dict, LORCoordinates, Sinogra
         norm = torch.ones(shape, dtype=torch.float32, device=device) if header["normalization_flag"] else None
         _lib.check(lib.sss_histogram_finish(_ptr(events), n, C.byref(L), C.byref(M), _ptr(counts), _ptr(last),
                                             float(header["duration"]), _ptr(prompts), _ptr(randoms), _ptr(norm), st))
-    torch.cuda.current_stream(device).synchronize()
-    _lib.check_status(int(status.item()))
+    _lib.check_status(int(status.item()))  # waits for the stream
     return prompts, randoms, norm
 
 
@@ -139,15 +138,14 @@ def inject_device(events: torch.Tensor, header: dict, LORCoordinates, slice_tabl
     lib = _lib.lib()
     ws = torch.empty(int(lib.sss_inject_workspace_size(n)), dtype=torch.uint8, device=device)
     out = torch.empty(n * (L.record_bytes + 4), dtype=torch.uint8, device=device)
-    count = torch.zeros(1, dtype=torch.int64, device=device)
-    status = torch.zeros(1, dtype=torch.int32, device=device)
+    result = torch.zeros(2, dtype=torch.int64, device=device)  # count and status (32 bits): one read-back
+    count, status = result[:1], result[1:]
     fac = torch.from_numpy(np.ascontiguousarray(factor, dtype=np.float32)).to(device)
     st = C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
     _lib.check(lib.sss_inject_scatters(_ptr(events), n, C.byref(L), C.byref(M), _ptr(scatters), _ptr(fac),
                                        _ptr(out), _ptr(count), _ptr(ws), ws.numel(), _ptr(status), st))
-    torch.cuda.current_stream(device).synchronize()
-    _lib.check_status(int(status.item()))
-    kept = int(count.item())
+    kept, state = result.cpu().tolist()
+    _lib.check_status(state)
     return out[: kept * (L.record_bytes + 4)], kept
 
 

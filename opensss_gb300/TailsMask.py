@@ -65,8 +65,7 @@ def tail_mask_device(volume, ImageSize, Geometry, SinogramCoordinates, SinogramI
         grid.ctypes.data_as(C.c_void_p), bounds.ctypes.data_as(C.c_void_p), _ptr(vol), int(bool(use_activity)), nr, nd,
         _ptr(g), _ptr(lor), _ptr(si), _ptr(pairs), npairs, nslices, int(AccelerationFactor or 1), acf, _ptr(out),
         _ptr(status), _ptr(ws), ws.numel(), C.c_void_p(st.cuda_stream)))
-    st.synchronize()
-    _lib.check_status(int(status.item()))
+    _lib.check_status(int(status.item()))  # waits for the stream
     return out
 
 
