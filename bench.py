@@ -291,42 +291,37 @@ def run_ours(args, rank, world, local_rank):
 
     if rank != 0:
         return
-    # ---- roofline of the dominant kernel.  The pair kernel reads, per
-    # (voxel of a walked leg, detector pair), the bins' TOF factors (4 B a
-    # bin) and the voxel's activity x length and distance (8 B): the per-unit
-    # bytes of the reference's TOF-table gather, taken from shared memory.
+    # ---- roofline of the dominant stage.  The pair stage adds, per (voxel of a
+    # walked leg, detector pair), the voxel's value to the counter of its TOF
+    # offset in shared memory: 8 bytes, read and written.  (The reference gathers
+    # 4 bytes a bin from its TOF table there.)
     pair_s = statistics.mean(pair_ms) / 1e3
     walked = stage[4] / pr.nr_bins if stage[4] > 0 else None  # (voxel, pair) terms of one step
-    alg_bytes = walked * (4 * pr.nr_bins + 8) if walked else None
+    alg_bytes = walked * 8 if walked else None
+    gather = walked * (4 * pr.nr_bins + 8) / pair_s / 1e9 if walked else None
     peaks = _probe_peaks()
     achieved = alg_bytes / pair_s / 1e9 if alg_bytes else None
-    # FP32 work of the weights: per term and bin one FMA into the bin's sum and
-    # one multiply of the running power (3 flops); SFU: 2^x of the two legs'
-    # attenuation terms per evaluated pair and scatter point
-    fp32_gflops = 3 * stage[4] / pair_s / 1e9 if stage[4] > 0 else None
+    # SFU: 2^x of the two legs' attenuation terms per evaluated pair and scatter point
     sfu_g = 2 * stage[5] / pair_s / 1e9 if stage[5] > 0 else None
-    roof = {"bound": "smem", "unit": "GB/s", "kernel": "pair_kernel", "achieved": achieved,
+    roof = {"bound": "smem", "unit": "GB/s", "kernel": "factor_kernel + hist_kernel", "achieved": achieved,
             "peak": peaks["smem"], "peak_source": "measured (sss_probe_smem_rate, this run)",
             "frac": achieved / peaks["smem"] if achieved and peaks["smem"] else None,
             "traffic": None,
             "traffic_note": "DRAM bytes come from an ncu capture only, not from this run; "
-                            "the TOF factors are read from shared memory, not DRAM",
+                            "the counters are in shared memory, not DRAM",
             "algorithmic_bytes_per_launch": alg_bytes,
-            "bytes_rule": "(4 B x bins + 8 B) per (voxel, detector pair) term walked",
+            "bytes_rule": "8 B (a counter read and written) per (voxel, detector pair) term walked; a scattered "
+                          "atomic of a warp occupies the shared memory 3.75 cycles, a plain access 1",
             "terms_per_launch": walked, "launch_ms": pair_s * 1e3,
-            "fp32_pipe": {"achieved_gflops": fp32_gflops, "peak_gflops": peaks["ffma"],
-                          "frac": fp32_gflops / peaks["ffma"] if fp32_gflops and peaks["ffma"] else None,
-                          "rule": "3 flops (FMA + power multiply) per (voxel, pair) term and bin",
-                          "peak_source": "measured (sss_probe_ffma_rate, FFMA2 chains, this run)"},
             "sfu": {"achieved_g_per_s": sfu_g, "peak_g_per_s": peaks["ex2"],
                     "frac": sfu_g / peaks["ex2"] if sfu_g and peaks["ex2"] else None,
                     "rule": "two 2^x per evaluated (pair, scatter point)",
                     "peak_source": "measured (sss_probe_ex2_rate, this run)"},
             "l2_reference_gather": {
-                "achieved": achieved, "peak": peaks["l2"], "unit": "GB/s",
-                "frac": achieved / peaks["l2"] if achieved and peaks["l2"] else None,
+                "achieved": gather, "peak": peaks["l2"], "unit": "GB/s",
+                "frac": gather / peaks["l2"] if gather and peaks["l2"] else None,
                 "peak_source": "measured (sss_probe_l2_rate, 32 MB L2-resident, this run)",
-                "note": "same bytes against the L2 load bandwidth a TOF-table gather would be bound by"},
+                "note": "(4 B x bins + 8 B) a term against the L2 load bandwidth a TOF-table gather would be bound by"},
             "weights_per_s": stage[4] / pair_s if stage[4] > 0 else None}
 
     # ---- CPU baseline (oracle port on the host cores) and the error against

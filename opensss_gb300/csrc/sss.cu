@@ -545,7 +545,7 @@ extern "C" int sss_tof_run(const sss_tof_problem* p, const double* points, int64
             }
             if (rc) return rc;
             if (g_timer.on) cudaEventRecord(g_timer.get(), st);
-            g_timer.launches += 2;
+            g_timer.launches += hist && !HL.unit ? 4 : 2;  // legs; factors, histogram, empty cells or the pairs
             g_timer.waves += 1;
         }
         first += npts;
